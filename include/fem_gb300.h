@@ -214,6 +214,12 @@ int fem_set_wait_limit(FemHandle* handle, int64_t nanoseconds);
                                         needs the 16-bit column offsets (FEM_TUNE_COMPACT_COLUMNS not 0); otherwise
                                         the direct loads run.  A copy that does not complete within the wait limit
                                         sets the timeout status that fem_get_stats reports. */
+#define FEM_TUNE_ONCHIP 17           /* the PCG that keeps a CTA's matrix rows in shared memory and its CG vectors in
+                                        registers, with one grid reduction per iteration: -1 (default) when the rows
+                                        fit (one scene, at most 1024 rows per SM) and none of the streaming kernel's
+                                        keys above was changed; 0 never; 1 whenever the rows fit (standard recurrence
+                                        and uncalibrated split only) */
+#define FEM_TUNE_ONCHIP_GRID 18      /* read-only: that kernel's grid, 0 while solves use the streaming kernel */
 int fem_set_tuning(FemHandle* handle, int32_t key, int64_t value);
 int fem_get_tuning(FemHandle* handle, int32_t key, int64_t* value);
 int fem_set_maxiter(FemHandle* handle, int32_t maxiter);

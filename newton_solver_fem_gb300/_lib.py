@@ -38,6 +38,8 @@ FEM_TUNE_UNIFORM_COLUMN_BLOCKS = 13
 FEM_TUNE_CG_VARIANT = 14
 FEM_TUNE_OPERATOR_BATCH = 15
 FEM_TUNE_OPERATOR_STAGE = 16
+FEM_TUNE_ONCHIP = 17
+FEM_TUNE_ONCHIP_GRID = 18
 
 FEM_TERM_SPRING = 1
 FEM_TERM_TET = 2

@@ -140,7 +140,7 @@ class _Substep(torch.autograd.Function):
         vb = torch.zeros_like(v_in) if v_out_bar is None else v_out_bar.contiguous().clone()
         qb[diff.fixed] = 0.0  # fixed outputs are overwritten by the restore
         vb[diff.fixed] = 0.0
-        vt = vb + dt * qb
+        vt = torch.add(vb, qb, alpha=dt)  # one rounding, as the device schedule's seed kernel
         rhs_bar = diff.solve(vt)
         if diff.after_backward_solve is not None:
             diff.after_backward_solve()
@@ -273,9 +273,10 @@ class DeviceRollout:
         lib = self.diff.lib
         total = 0
         for d in (self.diff, self.overlap):
-            v = ctypes.c_int64()
-            _lib.check(lib.fem_get_tuning(d.solver._handle, _lib.FEM_TUNE_GRID, ctypes.byref(v)))
-            total += int(v.value)
+            onchip, grid = ctypes.c_int64(), ctypes.c_int64()
+            _lib.check(lib.fem_get_tuning(d.solver._handle, _lib.FEM_TUNE_ONCHIP_GRID, ctypes.byref(onchip)))
+            _lib.check(lib.fem_get_tuning(d.solver._handle, _lib.FEM_TUNE_GRID, ctypes.byref(grid)))
+            total += int(onchip.value) or int(grid.value)
         sms = torch.cuda.get_device_properties(self.diff.device).multi_processor_count
         return total <= sms
 

@@ -10,6 +10,8 @@ PCG axes (``fem_set_tuning`` keys):
   reductions);
 * the CG recurrence -- ``FEM_TUNE_CG_VARIANT``: standard (two grid reductions
   per iteration) or single-reduction Chronopoulos-Gear;
+* where the matrix stays -- ``FEM_TUNE_ONCHIP``: the on-chip kernel, or the
+  streaming kernel with the axes above;
 * the matrix bytes held in L2 (``FEM_TUNE_L2_RESIDENT_BYTES``): the automatic
   rule (-2: the whole matrix when it fits in 60% of L2, else none) won every
   measurement, so candidates keep it.
@@ -55,19 +57,22 @@ AXES = {
     "threads": _lib.FEM_TUNE_CTA_THREADS,
     "cg_variant": _lib.FEM_TUNE_CG_VARIANT,
     "resident_bytes": _lib.FEM_TUNE_L2_RESIDENT_BYTES,
+    "onchip": _lib.FEM_TUNE_ONCHIP,
 }
-# every staging depth at every CTA size with the standard recurrence, plus the single-reduction
-# recurrence at the default shape
-DEFAULT_CANDIDATES = [dict(unroll=u, threads=t, cg_variant=0, resident_bytes=-2)
+# the on-chip kernel (the streaming kernel's first shape again where the rows do not fit), then the
+# streaming kernel: every staging depth at every CTA size with the standard recurrence, plus the
+# single-reduction recurrence at the default shape
+DEFAULT_CANDIDATES = [dict(unroll=4, threads=1024, cg_variant=0, resident_bytes=-2, onchip=1)] + \
+                     [dict(unroll=u, threads=t, cg_variant=0, resident_bytes=-2, onchip=0)
                       for t in (1024, 512, 256) for u in (4, 2, 1)] + \
-                     [dict(unroll=u, threads=1024, cg_variant=1, resident_bytes=-2) for u in (4, 2)]
+                     [dict(unroll=u, threads=1024, cg_variant=1, resident_bytes=-2, onchip=0) for u in (4, 2)]
 CACHE = Path(os.environ.get("FEM_GB300_TUNE_CACHE", Path.home() / ".cache" / "fem_gb300_tune.json"))
 
 
 def _key(solver) -> str:
     info = solver.matrix_info()
     name = torch.cuda.get_device_name(solver.device)
-    return f"{name}|P={solver.model.particle_count}|blocks={info['stored_blocks']}|S={solver.model.scene_count}"
+    return f"{name}|onchip|P={solver.model.particle_count}|blocks={info['stored_blocks']}|S={solver.model.scene_count}"
 
 
 def apply(solver, choice: dict) -> None:

@@ -34,10 +34,10 @@ struct DeviceGuard {
 };
 
 template <class F>
-void parallel_for(int64_t n, F&& fn) {
+void parallel_for(int64_t n, F&& fn, int64_t grain = 4096) {
     unsigned hw = std::thread::hardware_concurrency();
     int nt = (int)std::max(1u, std::min(hw == 0 ? 1u : hw, 32u));
-    if (n < 4096 || nt == 1) {
+    if (n < grain || nt == 1) {
         fn(0, n);
         return;
     }
@@ -340,6 +340,58 @@ int configure_launch(Handle& h) {
     std::vector<float> zeros(2 * 3 * (size_t)std::max(1, nseg), 0.0f);
     h.seg_part = upload_plain(zeros, h.launch_allocations, err);
     if (err != cudaSuccess) return cuda_status(err, &h);
+    return FEM_OK;
+}
+
+// The on-chip PCG's plan, tables and records, when the rows fit and the grid is co-resident.
+int plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vector<unsigned>& row_info,
+                const std::vector<int>& scol) {
+    Handle& h = b.h;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const fem::OnchipInput in{scol, slice_meta, row_info,
+                              [&](int grid) {
+                                  return split_slices(h.host_slice_cost, std::vector<double>(grid, 1.0),
+                                                      (h.nslices + grid - 1) / grid);
+                              },
+                              [&](int64_t n, std::function<void(int64_t, int64_t)> fn) {
+                                  parallel_for(n, fn, h.nsell < 200000 ? n + 1 : 2);  // threads only for much work
+                              }};
+    fem::OnchipPlan plan;
+    fem::onchip_plan(h, in, sms, plan);
+    if (plan.grid == 0) return FEM_OK;
+    bool resident = false;
+    cudaError_t e = fem::onchip_allow(plan, sms, &resident);
+    if (e != cudaSuccess) return cuda_status(e, &h);
+    if (!resident) return FEM_OK;
+    // one allocation for the tables and one for the records and partials (a small solver's construction
+    // is mostly allocations)
+    std::vector<unsigned char> blob;
+    auto put = [&](const auto& v) {
+        const size_t at = (blob.size() + 15) & ~(size_t)15, bytes = v.size() * sizeof(v[0]);
+        blob.resize(at + bytes);
+        if (bytes) std::memcpy(blob.data() + at, v.data(), bytes);
+        return at;
+    };
+    const size_t o_slice0 = put(plan.slice0), o_kres = put(plan.kres), o_ptr = put(plan.halo_ptr),
+                 o_halo = put(plan.halo), o_lcol = put(plan.lcol);
+    unsigned char* tables = b.upload(blob);
+    float4* work = b.alloc<float4>(6 * (size_t)h.P + 4 * (size_t)plan.grid);
+    if (b.status != FEM_OK) return b.status;
+    h.oc_slice0 = reinterpret_cast<int*>(tables + o_slice0);
+    h.oc_kres = reinterpret_cast<int2*>(tables + o_kres);
+    h.oc_halo_ptr = reinterpret_cast<int*>(tables + o_ptr);
+    h.oc_halo = reinterpret_cast<int*>(tables + o_halo);
+    h.oc_lcol = reinterpret_cast<unsigned short*>(tables + o_lcol);
+    h.oc_rec0 = work;
+    h.oc_rec1 = work + 3 * (size_t)h.P;
+    h.oc_part = reinterpret_cast<float*>(work + 6 * (size_t)h.P);
+    h.oc_grid = plan.grid;
+    h.oc_threads = plan.threads;
+    h.oc_hybrid = plan.hybrid;
+    h.oc_meet = plan.meet;
+    h.oc_smem = plan.smem;
     return FEM_OK;
 }
 
@@ -882,7 +934,7 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
     } else {
         h.dv = b.alloc<float>(3 * (size_t)P);
     }
-    h.barrier = b.alloc<unsigned>(1);
+    h.barrier = b.alloc<unsigned>(fem::kBarrierWords);
     h.status = b.alloc<int>(1);
     h.scene_stats = b.alloc<fem::SceneStats>(nscenes);
     h.cum_iters = b.alloc<long long>(nscenes);
@@ -908,6 +960,7 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
     for (int sl = 0; sl < h.nslices; ++sl)
         for (int l = 0; l < slice_meta[sl].y; ++l) h.host_slice_cost[sl] += row_nnz[slice_meta[sl].x + l] + 4;
     int code = configure_launch(h);
+    if (code == FEM_OK) code = plan_onchip(b, slice_meta, row_info, scol);
     if (code != FEM_OK) {
         g_error = h.last_error;
         fem_destroy(H);
@@ -1104,6 +1157,7 @@ int fem_prepare_tet_updates(FemHandle* H, const FemDesc* d, int32_t original_nod
     n.compact_cols = h.compact_cols;
     n.resident_pref = h.resident_pref;
     n.cg_variant = h.cg_variant;
+    n.onchip = h.onchip;
     n.operator_batch = h.operator_batch;
     n.operator_stage = h.operator_stage;
     n.cta_speed = h.cta_speed;  // speeds belong to CTA indices, so they carry over to the new split
@@ -1189,6 +1243,7 @@ int fem_refresh_topology(FemHandle* H, const FemDesc* d, float* q, float dt, voi
     n.compact_cols = h.compact_cols;
     n.resident_pref = h.resident_pref;
     n.cg_variant = h.cg_variant;
+    n.onchip = h.onchip;
     n.operator_batch = h.operator_batch;
     n.operator_stage = h.operator_stage;
     n.cta_speed = h.cta_speed;  // speeds belong to CTA indices, so they carry over to the new split
@@ -1300,6 +1355,10 @@ int fem_set_tuning(FemHandle* H, int32_t key, int64_t value) {
         if (value != 0 && value != 4 && value != 8) return set_error(FEM_ERR_BAD_ARG, "operator stage must be 0, 4 or 8");
         h.operator_stage = (int)value;
         return FEM_OK;
+    } else if (key == FEM_TUNE_ONCHIP) {
+        if (value < -1 || value > 1) return set_error(FEM_ERR_BAD_ARG, "on-chip PCG must be -1, 0 or 1");
+        h.onchip = (int)value;
+        return FEM_OK;  // its tables are laid out at construction
     } else if (key == FEM_TUNE_CG_VARIANT) {
         if (value != 0 && value != 1) return set_error(FEM_ERR_BAD_ARG, "CG variant must be 0 or 1");
         h.cg_variant = (int)value;
@@ -1347,6 +1406,8 @@ int fem_get_tuning(FemHandle* H, int32_t key, int64_t* value) {
         case FEM_TUNE_CG_VARIANT: *value = h.cg_variant; return FEM_OK;
         case FEM_TUNE_OPERATOR_BATCH: *value = h.operator_batch; return FEM_OK;
         case FEM_TUNE_OPERATOR_STAGE: *value = h.operator_stage; return FEM_OK;
+        case FEM_TUNE_ONCHIP: *value = h.onchip; return FEM_OK;
+        case FEM_TUNE_ONCHIP_GRID: *value = fem::onchip_in_use(h) ? h.oc_grid : 0; return FEM_OK;
         default: return set_error(FEM_ERR_BAD_ARG, "unknown tuning key");
     }
 }

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -12,6 +13,9 @@ namespace fem {
 
 constexpr int kSlice = 32;          // rows per SELL slice (one warp, thread per row)
 constexpr int kPcgMaxThreads = 1024;  // largest persistent PCG block (the launch bound)
+constexpr int kBarrierWords = 96;     // barrier counters of a handle, on lines of their own:
+constexpr int kOnchipBarrier = 32;    //   [0] the streaming PCG (cleared before each launch),
+constexpr int kOnchipTicket = 64;     //   the on-chip PCG's barrier and exit ticket (cleared by its last CTA)
 constexpr unsigned kFixedBit = 0x80000000u;  // row_info: fixed-node flag; low bits = row length
 
 // Device-side status bits (FemStats.status).
@@ -142,6 +146,7 @@ struct Handle {
     int tail_prefetch = 50;          // FEM_TUNE_TAIL_PREFETCH (percent of warps busy in the last round)
     int resident_pref = -1;          // resident row-state layout: -1 automatic, 0 none, 1 x/r/z, 2 x/r/z + inverse
     int cg_variant = 0;              // FEM_TUNE_CG_VARIANT: 0 standard CG, 1 single-reduction (Chronopoulos-Gear)
+    int onchip = -1;                 // FEM_TUNE_ONCHIP: -1 automatic, 0 off, 1 whenever the handle has a plan
     int operator_batch = 2;          // FEM_TUNE_OPERATOR_BATCH: block columns in flight per thread in fem_apply_operator
     int operator_stage = 4;          // FEM_TUNE_OPERATOR_STAGE: 0 direct loads, else block columns per bulk copy
     std::vector<double> cta_speed;   // calibrated SpMV speed per CTA index (cost units per ns)
@@ -299,6 +304,16 @@ struct Handle {
     int resident = 0;                       // row state resident in shared memory (see PcgArgs)
     float* dv = nullptr;
     bool dv_owned = true;
+    // on-chip PCG (fem_pcg_onchip.cu): launch shape and tables, oc_grid 0 when the rows do not fit
+    int oc_grid = 0, oc_threads = 0, oc_hybrid = 0, oc_meet = 0;
+    size_t oc_smem = 0;
+    int* oc_slice0 = nullptr;
+    int2* oc_kres = nullptr;
+    int* oc_halo_ptr = nullptr;
+    int* oc_halo = nullptr;
+    unsigned short* oc_lcol = nullptr;
+    float4 *oc_rec0 = nullptr, *oc_rec1 = nullptr;  // [3P] each: (z, p, t) records
+    float* oc_part = nullptr;                       // [2][oc_grid][8]
     // reductions / control
     int grid = 0;
     size_t pcg_smem = 0;
@@ -390,6 +405,34 @@ cudaError_t launch_export_triplets(Handle& h, float* values, cudaStream_t s);
 // it for one handle never invalidates another handle's launch (or a captured graph's).
 cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes);
 cudaError_t pcg_configure(Handle& h);
+// --- the on-chip PCG (fem_pcg_onchip.cu) ---
+struct OnchipInput {  // host copies of the SELL layout, and helpers
+    const std::vector<int>& scol;
+    const std::vector<int2>& slice_meta;
+    const std::vector<unsigned>& row_info;
+    std::function<std::vector<int>(int)> split;  // slices of each of n CTAs (n + 1 bounds)
+    std::function<void(int64_t, std::function<void(int64_t, int64_t)>)> parallel;
+};
+struct OnchipPlan {
+    int grid = 0, threads = 0, hybrid = 0, meet = 0;
+    size_t smem = 0;
+    std::vector<int> slice0, halo_ptr, halo;
+    std::vector<int2> kres;
+    std::vector<unsigned short> lcol;
+};
+void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& plan);
+cudaError_t onchip_allow(const OnchipPlan& plan, int sms, bool* resident);
+cudaError_t launch_pcg_onchip(Handle& h, float dt, int write_state, float* q_out, float* v_out, float* f_ws,
+                              cudaStream_t s, const float* solve_rhs, float* x_out, float tol, int maxiter,
+                              bool solve_warm);
+// Whether this handle's solves run on chip: it has a plan, and no launch option of the streaming
+// kernel was asked for (an explicit request, 1, wins over them; 0 turns it off).
+inline bool onchip_in_use(const Handle& h) {
+    if (h.oc_grid == 0 || h.onchip == 0 || h.cg_variant != 0 || h.balance != 0) return false;
+    return h.onchip == 1 || (h.pcg_threads == 0 && h.grid_cap == 0 && h.resident_pref == -1 && h.compact_cols == -1 &&
+                             h.l2_resident_bytes == -2 && h.spmv_unroll == 4 && h.tail_prefetch == 50 &&
+                             h.split_headroom == 0);
+}
 // Step mode (solve_rhs == nullptr): predictor, normalised PCG from the dv warm start, integration.
 // Solve mode: A x = solve_rhs from zero (projected at fixed rows), x written to x_out.
 // Solve mode with solve_warm: start from the packed h.x instead of zero (normalised like step mode).

@@ -31,8 +31,7 @@
 #include <mutex>
 #include <utility>
 
-#include "fem_internal.cuh"
-#include "fem_math.cuh"
+#include "fem_grid.cuh"
 
 namespace fem {
 namespace {
@@ -51,73 +50,10 @@ struct SceneState {
     int primed;  // single-reduction variant: the first SpMV (w0 = A u0) has been reduced
 };
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ int ld_relaxed_int(const int* p) {
-    int v;
-    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Grid barrier over a monotone counter (zeroed before the launch), entered by
-// one thread per CTA after a CTA or warp barrier has ordered the CTA's writes
-// before it.  The arrival is a release reduction, so those writes are visible
-// at GPU scope before it; the wait is an acquire load, so the other CTAs'
-// writes are visible after it.  The wait is bounded: it gives up after
-// limit_ns nanoseconds, or as soon as another CTA has given up, and returns 0.
-__device__ __forceinline__ int arrive_and_wait(unsigned* counter, unsigned nblocks, unsigned& epoch, int* status,
-                                               long long limit_ns) {
-    epoch += 1;
-    const unsigned target = epoch * nblocks;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-    const unsigned long long t0 = global_ns();
-    unsigned spins = 0;
-    while ((int)(ld_acquire(counter) - target) < 0) {  // wrap-safe: the counter only grows
-        if ((++spins & 63u) == 1u) {  // first spin, then every 64th
-            if ((ld_relaxed_int(status) & kStatusTimeout) != 0 || (long long)(global_ns() - t0) >= limit_ns) {
-                atomicOr(status, kStatusTimeout);
-                return 0;
-            }
-        }
-    }
-    return 1;
-}
-
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
-}
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
-    return v;
-}
-__device__ __forceinline__ float3 bmul(float4 a, float4 b, float c, float3 p) {
-    return f3(a.x * p.x + a.y * p.y + a.z * p.z, a.w * p.x + b.x * p.y + b.y * p.z, b.z * p.x + b.w * p.y + c * p.z);
-}
-
 __device__ __forceinline__ float3 minv_mul(const float* __restrict__ m, int row, float3 r) {
     const float* b = m + 9 * (size_t)row;
     return f3(b[0] * r.x + b[1] * r.y + b[2] * r.z, b[3] * r.x + b[4] * r.y + b[5] * r.z,
               b[6] * r.x + b[7] * r.y + b[8] * r.z);
-}
-
-__device__ __forceinline__ float3 load3(const float* p, int i) { return f3(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
-__device__ __forceinline__ void store3(float* p, int i, float3 v) {
-    p[3 * i] = v.x;
-    p[3 * i + 1] = v.y;
-    p[3 * i + 2] = v.z;
 }
 
 // Same expression at the owner and at every gathering neighbour, so the
@@ -551,13 +487,6 @@ __device__ __noinline__ void prefetch_last_round(const PcgArgs& a, const Smem& s
     prefetch_range(a.valC + e0, m * sizeof(float), lane);
     if (a.dcol != nullptr) prefetch_range(a.dcol + e0, m * sizeof(short), lane);
     else prefetch_range(a.scol + e0, m * sizeof(int), lane);
-}
-
-__device__ __forceinline__ float rhs_scale(float maximum) {
-    // kernels.py:1785-1793
-    float scale = 1.0f;
-    if (maximum > 0.0f && maximum < 1.0e-12f) scale = fminf(1.0f / maximum, 1.0e30f);
-    return scale;
 }
 
 template <int U, int CM, int V>
@@ -1194,6 +1123,8 @@ cudaError_t pcg_configure(Handle& h) {
 
 cudaError_t launch_pcg(Handle& h, float dt, int write_state, float* q_out, float* v_out, float* f_ws, cudaStream_t s,
                        const float* solve_rhs, float* x_out, float tol, int maxiter, bool solve_warm) {
+    if (onchip_in_use(h))
+        return launch_pcg_onchip(h, dt, write_state, q_out, v_out, f_ws, s, solve_rhs, x_out, tol, maxiter, solve_warm);
     PcgArgs a;
     a.valA = h.valA;
     a.valB = h.valB;

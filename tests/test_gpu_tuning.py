@@ -198,3 +198,54 @@ def test_handles_needing_different_pcg_shared_memory_launch_in_any_order():
     graph.replay()
     torch.cuda.synchronize()
     assert np.isfinite(to_np(s1.particle_q)).all()
+
+
+# Slice and launch-shape edges of the on-chip kernel: one partial slice, exactly one and just over one
+# slice (32 and 33 rows are not grid sizes; 27 and 36 straddle them), one CTA, a cluster, a grid with
+# whole and with partly resident rows, and rows enough for the wide variant.
+ONCHIP_SHAPES = [("hex", (1, 1, 1)), ("tet", (2, 2, 2)), ("hex", (3, 2, 2)), ("tet", (4, 4, 4)), ("hex", (5, 5, 4)),
+                 ("tet", (4, 4, 16)), ("hex", (9, 9, 9)), ("hex", (13, 12, 11)), ("tet", (17, 13, 11)),
+                 ("hex", (23, 17, 11)), ("hex", (33, 32, 31)), ("tet", (46, 43, 41)), ("hex", (43, 42, 41))]
+
+
+@pytest.mark.parametrize("element,cells", ONCHIP_SHAPES, ids=lambda v: v if isinstance(v, str) else "x".join(map(str, v)))
+def test_onchip_kernel_solves_the_streaming_kernels_system(element, cells):
+    """Same tight-tolerance substep from a deformed, moving start and a warm start, with a fixed face; the
+    bound is the launch variants' one, as the recurrences agree to float32 round-off.  The adjoint-style
+    solve from zero is held to the same bound, and repeated substeps are bit-identical."""
+    from gpu_helpers import make_pair
+
+    block = scenes.tet_block if element == "tet" else scenes.hex_block
+    x, el, mats, mass = block(*cells, 0.01, (0.0, 0.0, 0.0), 2e5, 0.4, 1000.0)
+    fixed = np.nonzero(np.isclose(x[:, 0], 0.0))[0].astype(np.int32)
+    elements = {"tets": el, "tet_materials": mats} if element == "tet" else {"hexes": el, "hex_materials": mats}
+    model, solver, _ = make_pair(x, mass, fixed=fixed, gravity=(0.0, 0.0, -9.81), with_oracle=False,
+                                 linear_solver_tolerance=1e-6, linear_solver_maxiter=200, **elements)
+    lib = _lib.load()
+    rng = np.random.default_rng(31)
+    q = torch.tensor((x + rng.normal(0.0, 2e-4, x.shape)).astype(np.float32), device="cuda")
+    v = torch.tensor(rng.normal(0.0, 0.05, x.shape).astype(np.float32), device="cuda")
+    warm = torch.tensor(rng.normal(0.0, 5e-3, x.shape).astype(np.float32), device="cuda")
+    rhs = torch.tensor((rng.normal(0.0, 1.0, x.shape) * mass[:, None]).astype(np.float32), device="cuda")
+
+    def run():
+        s0, s1 = model.state(), model.state()
+        s0.particle_q.copy_(q)
+        s0.particle_qd.copy_(v)
+        solver.refresh_tangent(s0.particle_q)
+        solver.velocity_increment.copy_(warm)
+        solver.step(s0, s1, None, None, 1.0 / 600.0)
+        y = torch.empty_like(rhs)
+        _lib.check(lib.fem_solve(solver._handle, rhs.data_ptr(), y.data_ptr(), 1e-6, 200, solver._stream()))
+        torch.cuda.synchronize()
+        assert solver.stats()["status"] == 0
+        return to_np(solver.velocity_increment), to_np(s1.particle_q), to_np(y)
+
+    assert setting(solver, _lib.FEM_TUNE_ONCHIP_GRID) > 0
+    got, again = run(), run()
+    _lib.check(lib.fem_set_tuning(solver._handle, _lib.FEM_TUNE_ONCHIP, 0))
+    assert setting(solver, _lib.FEM_TUNE_ONCHIP_GRID) == 0
+    ref = run()
+    for a, b, c in zip(got, again, ref):
+        np.testing.assert_array_equal(a, b)
+        assert rel_l2(a, c) < 1e-5
