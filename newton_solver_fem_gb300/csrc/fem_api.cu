@@ -722,12 +722,13 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
             slice_meta.push_back(make_int2((int)r0, n));
             slice_scene.push_back(s);
             slice_ptr.push_back(slice_ptr.back() + w);
+            h.slice_width = std::max(h.slice_width, w);
         }
     }
     h.nslices = (int)slice_meta.size();
     const int64_t nsell = (int64_t)slice_ptr.back() * fem::kSlice;
     h.nsell = nsell;
-    std::vector<int> sell_slot(nsell, -1), sell_row(nsell, -1), scol(nsell, 0), slot_sell(nnzb);
+    std::vector<int> sell_slot(nsell, -1), sell_row(nsell, -1), scol(nsell, 0);
     std::vector<unsigned> row_info(P);
     parallel_for(h.nslices, [&](int64_t lo, int64_t hi) {
         for (int64_t sl = lo; sl < hi; ++sl) {
@@ -743,7 +744,6 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
                     if (k < row_nnz[r]) {
                         int slot = bsr_offsets[r] + k;
                         sell_slot[e] = slot;
-                        slot_sell[slot] = (int)e;
                         scol[e] = bsr_columns[slot];
                     }
                 }
@@ -826,9 +826,12 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
     h.elem_force = b.alloc<float4>(4 * (size_t)T + 8 * (size_t)Hn + 3 * (size_t)Tri);
     h.q4 = b.alloc<float4>(P);
     h.v4 = b.alloc<float4>(P);
-    h.trip.a = b.alloc<float4>((size_t)ntrip);
-    h.trip.b = b.alloc<float4>((size_t)ntrip);
-    h.trip.c = b.alloc<float>((size_t)ntrip);
+    h.trip_map.constants = off_tet;
+    h.trip_map.tets = T;
+    h.trip_map.hexes = Hn;
+    h.trip.a = b.alloc<float4>((size_t)h.trip_map.stored());
+    h.trip.b = b.alloc<float4>((size_t)h.trip_map.stored());
+    h.trip.c = b.alloc<float>((size_t)h.trip_map.stored());
     h.trip_rows = b.upload(trip_rows);
     h.trip_cols = b.upload(trip_cols);
     // contributor lists keyed by SELL entry (empty for padding), so the
@@ -847,18 +850,15 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
             for (int64_t e = lo; e < hi; ++e) {
                 int slot = sell_slot[e];
                 if (slot >= 0)
-                    std::copy(contrib.begin() + slot_cptr[slot], contrib.begin() + slot_cptr[slot + 1],
-                              sell_contrib.begin() + sell_cptr[e]);
+                    for (int i = 0; i < slot_cptr[slot + 1] - slot_cptr[slot]; ++i)
+                        sell_contrib[sell_cptr[e] + i] = (int)h.trip_map.place(contrib[slot_cptr[slot] + i]);
             }
         });
         h.sell_cptr = b.upload(sell_cptr);
         h.sell_contrib = b.upload(sell_contrib);
     }
-    h.sell_slot = b.upload(sell_slot);
-    h.sell_row = b.upload(sell_row);
     h.bsr_offsets = b.upload(bsr_offsets);
     h.bsr_columns = b.upload(bsr_columns);
-    h.slot_sell = b.upload(slot_sell);
     h.valA = b.alloc<float4>(nsell);
     h.valB = b.alloc<float4>(nsell);
     h.valC = b.alloc<float>(nsell);

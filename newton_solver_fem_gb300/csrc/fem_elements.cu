@@ -7,8 +7,8 @@
 //                     and soft contacts, ground, gravity, damping, and the h-scaled sum in the
 //                     reference's term order
 //   constant_blocks   mass + spring diagonal, spring off-diagonal and lumped triangle blocks
-//   tet_tangent       16 PSD blocks per tet (per-tet factors staged in shared memory)
-//   hex_tangent       64 PSD blocks per hex (Gauss-point data computed once per element)
+//   tet_tangent       the 10 blocks on and above the diagonal of a tet's PSD matrix
+//   hex_tangent       the 36 of a hex's (Gauss-point data computed once per element)
 // No float atomics anywhere: every sum runs in a fixed order.
 #include <climits>
 
@@ -494,13 +494,19 @@ __global__ void constant_tri_kernel(int Tri, const float4* __restrict__ pose, co
     for (int c = 0; c < 3; ++c) store_block(vals, trip_off + 3 * (int64_t)e + c, o);
 }
 
+// Pair u of the ten a <= b of 0..3: (0,0) (0,1) (0,2) (0,3) (1,1) (1,2) (1,3) (2,2) (2,3) (3,3).
+__device__ __forceinline__ void upper_pair(int u, int& a, int& b) {
+    a = u < 4 ? 0 : (u < 7 ? 1 : (u < 9 ? 2 : 3));
+    b = a + u - (a == 0 ? 0 : (a == 1 ? 4 : (a == 2 ? 7 : 9)));
+}
+
 constexpr int kTetTangentThreads = 128;
 constexpr int kTetFactor = 40;
 
 // Reference kernels.py:635-850.  Phase 1: one thread per tet computes the
 // per-tet factors (F dm_a, dJ/dx_a, dm_a and three coefficients) into shared
-// memory.  Phase 2: 16 consecutive threads write the 16 blocks of a tet, so
-// the 576-byte block run of each element is written contiguously.
+// memory.  Phase 2: 10 consecutive threads write the 10 blocks a <= b of a tet,
+// so the block run of each element is written contiguously.
 __global__ void __launch_bounds__(kTetTangentThreads) tet_tangent_kernel(
     int T, const int4* __restrict__ idx, const float* __restrict__ pose, const float* __restrict__ mat,
     const float* __restrict__ mu_scale, const float4* __restrict__ q4, float lo, float hi, float dt, int64_t trip_off,
@@ -556,16 +562,16 @@ __global__ void __launch_bounds__(kTetTangentThreads) tet_tangent_kernel(
     }
     __syncthreads();
     float scale = dt * dt;
-#pragma unroll 4
-    for (int m = 0; m < 16; ++m) {
+#pragma unroll 2
+    for (int m = 0; m < 10; ++m) {
         int b = lt + kTetTangentThreads * m;
-        int le = b >> 4, ab = b & 15;
+        int le = b / 10, ab = b - 10 * le;
         int te = blockIdx.x * kTetTangentThreads + le;
         if (te >= T) continue;
         const float* f = sm[le];
         float mode = f[39];
         if (mode == 2.0f) continue;
-        const int64_t ti = trip_off + 16 * (int64_t)te + ab;
+        const int64_t ti = trip_off + 10 * (int64_t)te + ab;
         float o[9];
         if (mode == 1.0f) {
 #pragma unroll
@@ -573,7 +579,8 @@ __global__ void __launch_bounds__(kTetTangentThreads) tet_tangent_kernel(
             store_block(vals, ti, o);
             continue;
         }
-        int a = ab >> 2, bb = ab & 3;
+        int a, bb;
+        upper_pair(ab, a, bb);
         float3 Fa = f3(f[3 * a], f[3 * a + 1], f[3 * a + 2]);
         float3 Fb = f3(f[3 * bb], f[3 * bb + 1], f[3 * bb + 2]);
         float3 Ja = f3(f[12 + 3 * a], f[13 + 3 * a], f[14 + 3 * a]);
@@ -609,15 +616,16 @@ __global__ void __launch_bounds__(kTetTangentThreads) tet_tangent_kernel(
 //   phase 1  one thread per (hex, point) forms gN_a, F, the clamp, cof F and the eight 9-float
 //            records r of its point (no work repeated across lanes);
 //   phase 2  one thread per 2x2 tile of blocks on or above the block diagonal (10 tiles per
-//            hex) sums its four blocks over the 8 points; a tile off the diagonal also gives
-//            the four transposed blocks below it (K_ba = K_ab^T term by term, so A is
-//            exactly symmetric).  Threads are tile-major (16 hexes per tile), so a quarter
+//            hex) sums its four blocks over the 8 points (K_ba = K_ab^T term by term, so the
+//            blocks below the diagonal are not formed and A is exactly symmetric).  Threads are tile-major (16 hexes per tile), so a quarter
 //            warp reads 8 hexes' records in 8 distinct bank groups and a diagonal tile's half
 //            warp skips its column-side loads;
-//   phase 3  the 64 blocks per hex are staged in shared memory in the triplet planes' layout
-//            (hexes padded apart so the staging stores are conflict-free) and written out by
-//            bulk asynchronous copies (cp.async.bulk), one per hex and plane.
-constexpr int kTanHex = 16;
+//   phase 3  the 36 blocks per hex are staged in shared memory in the triplet planes' layout (block by
+//            block over the group's 16 hexes, so a half warp stores one run) and written out by one
+//            bulk asynchronous copy (cp.async.bulk) per plane.
+// 48^3 hexes: 105 us writing all 64 blocks a hex, 80 writing 36 (143 MB); what bounds it is shared
+// memory (about 2,000 wavefronts a CTA, 47 us) and issue (about 7,500 instructions, 44 us) together.
+constexpr int kTanHex = kHexGroup;
 constexpr int kTanTiles = 10;
 constexpr int kTanThreads = kTanHex * kTanTiles;
 constexpr int kTanRec = 12;                                // words per record (9 used)
@@ -625,23 +633,15 @@ constexpr int kTanPointStride = 8 * kTanRec + 4;           // padded: the 8 poin
 constexpr int kTanHexStride = 8 * kTanPointStride + 4;     // padded: hexes of a warp in distinct banks
 constexpr int kTanTabStride = 28;                          // padded Gauss table row
 constexpr int kTanSgnStride = 9;                           // padded per-hex row of point signs
-constexpr int kTanOut4Stride = 65;                         // staged float4 blocks per hex (padded)
-constexpr int kTanOut1Stride = 68;                         // staged last-entry floats per hex (padded)
+constexpr int kTanBlocks = 36;                             // blocks a <= b of a hex
 constexpr size_t kTanRecBytes = sizeof(float) * kTanHex * kTanHexStride;
-constexpr size_t kTanOutA = 0, kTanOutB = 16 * kTanOut4Stride * kTanHex, kTanOutC = 2 * kTanOutB;
+constexpr size_t kTanOutA = 0, kTanOutB = 16 * kTanBlocks * kTanHex, kTanOutC = 2 * kTanOutB;
 constexpr size_t kTanXOff = kTanRecBytes;
 constexpr size_t kTanSgnOff = kTanXOff + 16 * 8 * kTanHex;
 constexpr size_t kTanTabOff = kTanSgnOff + 16 * kTanSgnStride * kTanHex;
 constexpr size_t kTanSmemBytes = kTanTabOff + sizeof(float) * 8 * kTanTabStride;
-static_assert(kTanOutC + 4 * kTanOut1Stride * kTanHex <= kTanRecBytes, "output staging reuses the record area");
-static_assert((16 * kTanOut4Stride) % 16 == 0 && (4 * kTanOut1Stride) % 16 == 0, "16-byte bulk copy sources");
+static_assert(kTanOutC + 4 * kTanBlocks * kTanHex <= kTanRecBytes, "output staging reuses the record area");
 static_assert(kTanRec % 4 == 0 && kTanPointStride % 4 == 0 && kTanHexStride % 4 == 0, "16-byte records");
-
-__device__ __forceinline__ void tan_tile_rows(int t, int& A, int& B) {
-    // (0,0) (0,1) (0,2) (0,3) (1,1) (1,2) (1,3) (2,2) (2,3) (3,3)
-    A = t < 4 ? 0 : (t < 7 ? 1 : (t < 9 ? 2 : 3));
-    B = A + t - (A == 0 ? 0 : (A == 1 ? 4 : (A == 2 ? 7 : 9)));
-}
 
 __device__ __forceinline__ void tan_load_record(const float* p, float (&r)[9]) {
     const float4 v0 = reinterpret_cast<const float4*>(p)[0];
@@ -823,7 +823,7 @@ __global__ void __launch_bounds__(kTanThreads, 4) hex_tangent_kernel(int H, cons
     // phase 2
     const int tile = tid / kTanHex, hl = tid - tile * kTanHex;
     int A, B;
-    tan_tile_rows(tile, A, B);
+    upper_pair(tile, A, B);
     const int a0 = 2 * A, b0 = 2 * B;
     float K[4][9];
     if (any_neg)
@@ -840,38 +840,27 @@ __global__ void __launch_bounds__(kTanThreads, 4) hex_tangent_kernel(int H, cons
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
+            if (A == B && i > j) continue;  // below the diagonal
             const float* k = K[2 * i + j];
-            const int blk = 8 * (a0 + i) + (b0 + j);
-            s_A[hl * kTanOut4Stride + blk] = make_float4(k[0], k[1], k[2], k[3]);
-            s_B[hl * kTanOut4Stride + blk] = make_float4(k[4], k[5], k[6], k[7]);
-            s_C[hl * kTanOut1Stride + blk] = k[8];
-            if (A != B) {
-                const int tr = 8 * (b0 + j) + (a0 + i);
-                s_A[hl * kTanOut4Stride + tr] = make_float4(k[0], k[3], k[6], k[1]);
-                s_B[hl * kTanOut4Stride + tr] = make_float4(k[4], k[7], k[2], k[5]);
-                s_C[hl * kTanOut1Stride + tr] = k[8];
-            }
+            const int a = a0 + i, u = a * 8 - a * (a - 1) / 2 + (b0 + j - a);
+            s_A[u * kTanHex + hl] = make_float4(k[0], k[1], k[2], k[3]);
+            s_B[u * kTanHex + hl] = make_float4(k[4], k[5], k[6], k[7]);
+            s_C[u * kTanHex + hl] = k[8];
         }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // staged blocks visible to the bulk copies
     __syncthreads();
-    const int nh = (int)min((int64_t)kTanHex, (int64_t)H - h0);
-    const int64_t base = trip_off + 64 * h0;
-    float* c_dst = vals.c + base;
-    const bool c_bulk = (reinterpret_cast<uintptr_t>(c_dst) & 15) == 0;
-    const int copies = c_bulk ? 3 * nh : 2 * nh;  // thread k copies plane k % 3 (or % 2) of hex k / 3 (or / 2)
-    if (tid < copies) {
-        const int per = c_bulk ? 3 : 2, hx = tid / per, plane = tid - hx * per;
-        if (plane == 0)
-            bulk_store_s2g(vals.a + base + 64 * hx, s_A + hx * kTanOut4Stride, 64 * 16);
-        else if (plane == 1)
-            bulk_store_s2g(vals.b + base + 64 * hx, s_B + hx * kTanOut4Stride, 64 * 16);
+    // the planes are padded to whole groups and start on 16 bytes
+    if (tid < 3) {
+        const int64_t base = trip_off + kTanBlocks * h0;
+        if (tid == 0)
+            bulk_store_s2g(vals.a + base, s_A, 16 * kTanBlocks * kTanHex);
+        else if (tid == 1)
+            bulk_store_s2g(vals.b + base, s_B, 16 * kTanBlocks * kTanHex);
         else
-            bulk_store_s2g(c_dst + 64 * hx, s_C + hx * kTanOut1Stride, 64 * 4);
+            bulk_store_s2g(vals.c + base, s_C, 4 * kTanBlocks * kTanHex);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory stays until read
     }
-    if (!c_bulk)
-        for (int i = tid; i < nh * 64; i += kTanThreads) c_dst[i] = s_C[(i >> 6) * kTanOut1Stride + (i & 63)];
-    if (tid < copies) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory stays until read
 }
 
 }  // namespace
@@ -1021,7 +1010,7 @@ cudaError_t launch_element_tangent(Handle& h, float dt, cudaStream_t s) {
         if (err != cudaSuccess) return err;
         hex_tangent_kernel<<<blocks_for(h.H, kTanHex), kTanThreads, kTanSmemBytes, s>>>(
             h.H, h.hex_idx, h.hex_invJ, h.hex_detw, h.hex_mat, h.q4, h.min_stretch, h.max_stretch, dt,
-            tet_off + 16 * (int64_t)h.T, h.trip);
+            h.trip_map.hex_start(), h.trip);
     }
     return cudaGetLastError();
 }

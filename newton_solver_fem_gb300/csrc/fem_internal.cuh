@@ -32,6 +32,38 @@ struct TripletPlanes {
     float* c = nullptr;
 };
 
+// Where the planes hold a triplet.  Element matrices are exactly symmetric (the kernels form K_ba as the
+// transpose of K_ab, term by term), so only the blocks a <= b are stored: 10 of a tet's 16 and 36 of a
+// hex's 64; a block below the diagonal is read transposed.  That is 0.56 of the bytes the tangent
+// kernels write and the assembly reads.  The hexes are stored in groups of 16 (one tangent CTA), block
+// by block over the group's hexes: a CTA's output is one run per plane, and a slice's rows, which touch
+// consecutive hexes at a block, read consecutive entries.
+constexpr int kHexGroup = 16;
+struct TripletMap {
+    int64_t constants = 0;  // [P | 2S | 3Tri], stored as they are
+    int64_t tets = 0, hexes = 0;
+    __host__ __device__ __forceinline__ int64_t hex_start() const { return (constants + 10 * tets + 3) & ~(int64_t)3; }
+    __host__ __device__ __forceinline__ int64_t stored() const {
+        return hex_start() + 36 * kHexGroup * ((hexes + kHexGroup - 1) / kHexGroup);
+    }
+    // place << 1 | transposed of triplet t
+    __host__ __device__ __forceinline__ unsigned place(int64_t t) const {
+        int64_t at = t;
+        unsigned flip = 0;
+        if (t >= constants) {
+            const bool hex = t >= constants + 16 * tets;
+            const int n = hex ? 8 : 4;
+            const int64_t k = t - constants - (hex ? 16 * tets : 0), e = k / (n * n);
+            const int ab = (int)(k % (n * n)), a = ab / n, b = ab % n, lo = a < b ? a : b, hi = a < b ? b : a;
+            const int u = lo * n - lo * (lo - 1) / 2 + (hi - lo);
+            flip = a > b;
+            at = hex ? hex_start() + (e / kHexGroup) * (36 * kHexGroup) + u * kHexGroup + e % kHexGroup
+                     : constants + 10 * e + u;
+        }
+        return (unsigned)(at << 1) | flip;
+    }
+};
+
 #ifdef __CUDACC__
 __device__ __forceinline__ void store_block(const TripletPlanes& t, int64_t i, const float* v) {
     t.a[i] = make_float4(v[0], v[1], v[2], v[3]);
@@ -128,7 +160,7 @@ struct Handle {
     // sizes
     int P = 0, T = 0, H = 0, S = 0, Tri = 0, nfixed = 0, nscenes = 1;
     int64_t ntrip = 0, nnzb = 0, nsell = 0;
-    int nslices = 0;
+    int nslices = 0, slice_width = 0;  // slices, widest slice's block columns
     // options
     float dt = 0.f, min_stretch = 0.f, max_stretch = 0.f;
     int has_ground = 0;
@@ -267,13 +299,12 @@ struct Handle {
     float4* q4 = nullptr;
     float4* v4 = nullptr;
     // assembly
-    TripletPlanes trip;           // [ntrip] blocks
-    int* sell_slot = nullptr;     // [nsell] canonical slot or -1
+    TripletPlanes trip;           // [trip_map.stored()] blocks
+    TripletMap trip_map;
     int* sell_cptr = nullptr;     // [nsell+1] contributor range of each SELL entry
-    int* sell_contrib = nullptr;  // triplet ids, ascending within each entry
+    int* sell_contrib = nullptr;  // places of the triplets (TripletMap::place, unsigned), in triplet order in each entry
     int* bsr_offsets = nullptr;   // [P+1]
     int* bsr_columns = nullptr;   // [nnzb]
-    int* slot_sell = nullptr;     // [nnzb] canonical slot -> SELL entry
     int* trip_rows = nullptr;     // [ntrip] (export only)
     int* trip_cols = nullptr;
     // SELL matrix
@@ -290,7 +321,6 @@ struct Handle {
     int* slice_ptr = nullptr;
     int2* slice_meta = nullptr;
     int* slice_scene = nullptr;
-    int* sell_row = nullptr;  // [nsell] row of entry (or -1 for lanes past the slice)
     unsigned* row_info = nullptr;
     float* minv = nullptr;  // [P*9]
     // CG

@@ -202,7 +202,7 @@ __global__ void contrib_count_kernel(int P, int T, const int* __restrict__ diag_
     }
 }
 
-__global__ void contrib_scatter_kernel(int P, int T, const int* __restrict__ diag_entry,
+__global__ void contrib_scatter_kernel(int P, int T, TripletMap map, const int* __restrict__ diag_entry,
                                        const int* __restrict__ active, const int* __restrict__ slots,
                                        const int* __restrict__ start, int* __restrict__ count,
                                        int* __restrict__ contrib) {
@@ -216,7 +216,7 @@ __global__ void contrib_scatter_kernel(int P, int T, const int* __restrict__ dia
     }
     if (entry < 0) return;
     const int pos = atomicSub(count + entry, 1) - 1;
-    contrib[start[entry] + pos] = (int)t;
+    contrib[start[entry] + pos] = (int)map.place(t);  // streaming handles hold no springs or triangles
 }
 
 // Ascending order inside each segment [start[i], start[i+1]) (insertion sort; segments are short).
@@ -448,7 +448,7 @@ int streaming_update(Handle& h, const FemDesc* d, const float* q, const int* sou
                                                                h.entry_count);
     ok(cudaGetLastError());
     ok(launch_exclusive_scan(h.entry_count, h.sell_cptr, (int)h.nsell, h.scan_part, s));
-    contrib_scatter_kernel<<<blocks_for(nkeys, 256), 256, 0, s>>>(P, T, h.diag_entry, h.st_active, h.st_slot,
+    contrib_scatter_kernel<<<blocks_for(nkeys, 256), 256, 0, s>>>(P, T, h.trip_map, h.diag_entry, h.st_active, h.st_slot,
                                                                  h.sell_cptr, h.entry_count, h.sell_contrib);
     sort_segments_kernel<<<blocks_for(h.nsell, 256), 256, 0, s>>>(h.nsell, h.sell_cptr, h.sell_contrib);
     // node incidence of the element-force gather (every corner slot, ascending)
