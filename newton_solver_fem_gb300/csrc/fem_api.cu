@@ -375,9 +375,11 @@ int plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vect
         return at;
     };
     const size_t o_slice0 = put(plan.slice0), o_kres = put(plan.kres), o_ptr = put(plan.halo_ptr),
-                 o_halo = put(plan.halo), o_lcol = put(plan.lcol);
+                 o_halo = put(plan.halo), o_lcol = put(plan.lcol), o_team = put(plan.team);
     unsigned char* tables = b.upload(blob);
-    float4* work = b.alloc<float4>(6 * (size_t)h.P + 4 * (size_t)plan.grid);
+    // records, then the teams' counters, then partials
+    const size_t counters = (size_t)h.nscenes * fem::kTeamBarrierBytes / sizeof(float4);
+    float4* work = b.alloc<float4>(6 * (size_t)h.P + 8 + counters + 4 * (size_t)plan.grid);
     if (b.status != FEM_OK) return b.status;
     h.oc_slice0 = reinterpret_cast<int*>(tables + o_slice0);
     h.oc_kres = reinterpret_cast<int2*>(tables + o_kres);
@@ -386,7 +388,10 @@ int plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vect
     h.oc_lcol = reinterpret_cast<unsigned short*>(tables + o_lcol);
     h.oc_rec0 = work;
     h.oc_rec1 = work + 3 * (size_t)h.P;
-    h.oc_part = reinterpret_cast<float*>(work + 6 * (size_t)h.P);
+    h.oc_team = reinterpret_cast<int4*>(tables + o_team);
+    float4* line = work + ((6 * (size_t)h.P + 7) & ~(size_t)7);  // 128-byte lines
+    h.oc_barrier = reinterpret_cast<unsigned*>(line);
+    h.oc_part = reinterpret_cast<float*>(line + counters);
     h.oc_grid = plan.grid;
     h.oc_threads = plan.threads;
     h.oc_hybrid = plan.hybrid;
@@ -934,7 +939,7 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
     } else {
         h.dv = b.alloc<float>(3 * (size_t)P);
     }
-    h.barrier = b.alloc<unsigned>(fem::kBarrierWords);
+    h.barrier = b.alloc<unsigned>(1);
     h.status = b.alloc<int>(1);
     h.scene_stats = b.alloc<fem::SceneStats>(nscenes);
     h.cum_iters = b.alloc<long long>(nscenes);

@@ -12,10 +12,8 @@
 namespace fem {
 
 constexpr int kSlice = 32;          // rows per SELL slice (one warp, thread per row)
+constexpr int kTeamBarrierBytes = 256;  // a team's counters (fem_pcg_onchip.cu)
 constexpr int kPcgMaxThreads = 1024;  // largest persistent PCG block (the launch bound)
-constexpr int kBarrierWords = 96;     // barrier counters of a handle, on lines of their own:
-constexpr int kOnchipBarrier = 32;    //   [0] the streaming PCG (cleared before each launch),
-constexpr int kOnchipTicket = 64;     //   the on-chip PCG's barrier and exit ticket (cleared by its last CTA)
 constexpr unsigned kFixedBit = 0x80000000u;  // row_info: fixed-node flag; low bits = row length
 
 // Device-side status bits (FemStats.status).
@@ -338,6 +336,8 @@ struct Handle {
     int oc_grid = 0, oc_threads = 0, oc_hybrid = 0, oc_meet = 0;
     size_t oc_smem = 0;
     int* oc_slice0 = nullptr;
+    int4* oc_team = nullptr;
+    unsigned* oc_barrier = nullptr;  // per scene: barrier counter and exit ticket, zero between launches
     int2* oc_kres = nullptr;
     int* oc_halo_ptr = nullptr;
     int* oc_halo = nullptr;
@@ -448,6 +448,7 @@ struct OnchipPlan {
     size_t smem = 0;
     std::vector<int> slice0, halo_ptr, halo;
     std::vector<int2> kres;
+    std::vector<int4> team;
     std::vector<unsigned short> lcol;
 };
 void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& plan);

@@ -1,5 +1,6 @@
-// Persistent PCG for one scene whose rows are few enough that a CTA can keep its share on chip:
-// the matrix rows in shared memory and the CG vectors in registers, for the whole solve.
+// Persistent PCG for scenes whose rows are few enough that a CTA can keep its share on chip:
+// the matrix rows in shared memory and the CG vectors in registers, for the whole solve.  Several scenes
+// run as independent teams of CTAs in one launch, each with its own barrier and its own end.
 //
 // The streaming kernel (fem_pcg.cu) reads the matrix from L2 or DRAM every iteration and meets two
 // grid barriers; below about 100,000 nodes neither the bytes nor the operations bound it but the
@@ -88,6 +89,9 @@ __host__ __device__ __forceinline__ OcLayout oc_layout(int ns, int parts, int nh
 }
 __host__ __device__ __forceinline__ int oc_parts(int warps, int ns) { return ns > 0 ? max(1, warps / ns) : 1; }
 
+constexpr int kTeamWords = 64, kTeamTicket = 32;  // counter and ticket on lines of their own
+static_assert(kTeamWords * sizeof(unsigned) == kTeamBarrierBytes, "the host's allocation");
+
 struct OcArgs {
     const float4* __restrict__ valA;
     const float4* __restrict__ valB;
@@ -98,6 +102,7 @@ struct OcArgs {
     const unsigned* __restrict__ row_info;
     const float* __restrict__ minv;
     const int* __restrict__ slice0;    // [grid+1] first slice of each CTA
+    const int4* __restrict__ team;     // [grid] (first CTA, CTAs, scene, -) of the CTA's team
     const int2* __restrict__ kres;     // [nslices] (block columns in shared memory, the first one's place there)
     const int* __restrict__ halo_ptr;  // [grid+1]
     const int* __restrict__ halo;      // halo columns (node ids), per CTA ascending
@@ -116,8 +121,7 @@ struct OcArgs {
     float4* rec0;  // [3P] records (z, p, t), two alternating buffers
     float4* rec1;
     float* part;  // [2][grid][8]
-    unsigned* barrier;
-    unsigned* ticket;
+    unsigned* barrier;  // [scenes][kTeamWords] a team's barrier counter and exit ticket
     int* status;
     SceneStats* scene_stats;
     long long* cum_iters;
@@ -209,7 +213,7 @@ __device__ __forceinline__ float3 product_part(const OcArgs& a, const Share<kReg
 // distributed shared memory, one hardware cluster barrier per reduction: 1.0 us with 16 CTAs, the
 // exchange of records through L2 included, against 1.7 us for a counter barrier of as many CTAs), or
 // as a cooperative grid around a counter in global memory (2.4 us with 152).
-enum Meet { kAlone, kCluster, kGrid };
+enum Meet { kAlone, kCluster, kGrid, kTeams };  // kTeams: several such grids in one launch, one per scene
 
 __device__ __forceinline__ void store_remote(const float* p, unsigned rank, float v) {
     const unsigned local = static_cast<unsigned>(__cvta_generic_to_shared(p));
@@ -236,7 +240,7 @@ __device__ __forceinline__ float fold_groups(float acc, int c) {
 // then the CTAs' totals; lane 0 runs upd(totals).  Entered by the whole CTA; false after a wait that
 // ran out (kGrid only).
 template <Meet kMeet, bool kMax, class Update>
-__device__ __forceinline__ bool reduce8(const OcArgs& a, float (&v)[8], int ns, float* red, float* box,
+__device__ __forceinline__ bool reduce8(const OcArgs& a, int4 team, float (&v)[8], int ns, float* red, float* box,
                                         unsigned& epoch, int* s_ok, Update upd) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = lane & 7;
@@ -278,12 +282,12 @@ __device__ __forceinline__ bool reduce8(const OcArgs& a, float (&v)[8], int ns, 
         }
     }
     if (warp == 0) {
-        if (kMeet == kGrid) {
-            const int G = gridDim.x;
-            float* buf = a.part + (size_t)(epoch & 1u) * G * 8;
-            if (lane < 8) buf[blockIdx.x * 8 + lane] = acc;
+        if (kMeet == kGrid || (kMeet == kTeams && team.y > 1)) {
+            const int G = team.y;
+            float* buf = a.part + ((size_t)(epoch & 1u) * gridDim.x + team.x) * 8;
+            if (lane < 8) buf[(blockIdx.x - team.x) * 8 + lane] = acc;
             __syncwarp();
-            if (lane == 0) ok = arrive_and_wait(a.barrier, G, epoch, a.status, a.limit_ns);
+            if (lane == 0) ok = arrive_and_wait(a.barrier + team.z * kTeamWords, G, epoch, a.status, a.limit_ns);
             ok = __shfl_sync(0xffffffffu, ok, 0);
             epoch = __shfl_sync(0xffffffffu, epoch, 0);
             if (ok) {  // lane: half (lane & 1) of the records of CTAs (lane >> 1), (lane >> 1) + 16, ...
@@ -338,6 +342,8 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
     __shared__ OcState st;
     __shared__ int s_ok;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+    // a constant of the launch where there is one team (its registers cost the 64-register variant 9%)
+    const int4 team = kMeet == kTeams ? a.team[blockIdx.x] : make_int4(0, (int)gridDim.x, 0, 0);
     const int first = a.slice0[blockIdx.x], ns = a.slice0[blockIdx.x + 1] - first;
     const int h0 = a.halo_ptr[blockIdx.x], nhalo = a.halo_ptr[blockIdx.x + 1] - h0;
     const int Q = oc_parts(W, ns), rows = ns * kSlice;
@@ -542,7 +548,7 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
         publish(a.rec0);
         float v[8] = {dot3(r, r), dot3(r, z), dot3(rhs, rhs), 0.f, 0.f, 0.f, 0.f,
                       fmaxf(fabsf(rhs.x), fmaxf(fabsf(rhs.y), fabsf(rhs.z)))};
-        ok = reduce8<kMeet, true>(a, v, ns, red, box, epoch, &s_ok, [&](const float* T) {
+        ok = reduce8<kMeet, true>(a, team, v, ns, red, box, epoch, &s_ok, [&](const float* T) {
             if (T[7] == 0.0f) {  // b = 0: the warm start is cleared (x = 0 solves it)
                 const float none[8] = {0.f, 0.f, T[2], 0.f, 0.f, 0.f, 0.f, 0.f};
                 start(none);
@@ -564,7 +570,7 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
             const float3 b = rhs * scale;
             publish(a.rec0);
             float v[8] = {dot3(r, r), dot3(r, z), dot3(b, b), 0.f, 0.f, 0.f, 0.f, 0.f};
-            ok = reduce8<kMeet, false>(a, v, ns, red, box, epoch, &s_ok, start);
+            ok = reduce8<kMeet, false>(a, team, v, ns, red, box, epoch, &s_ok, start);
         }
     }
 
@@ -593,7 +599,7 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
         publish((it & 1) ? a.rec0 : a.rec1);
         {
             float v[8] = {dot3(p, s), dot3(z, s), dot3(tt, s), dot3(r, z), dot3(r, r), dot3(r, s), dot3(s, s), 0.f};
-            ok = reduce8<kMeet, false>(a, v, ns, red, box, epoch, &s_ok, [&](const float* T) {
+            ok = reduce8<kMeet, false>(a, team, v, ns, red, box, epoch, &s_ok, [&](const float* T) {
                 const float rz = T[3], rr = T[4], alpha = rz / T[0];
                 const float rz1 = quadratic(T[2], -2.0f * T[1], rz, alpha);
                 const float rr1 = quadratic(T[6], -2.0f * T[5], rr, alpha);
@@ -615,7 +621,7 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
             const float a1 = st.alpha;
             const float3 r1 = f3(fmaf(-a1, s.x, r.x), fmaf(-a1, s.y, r.y), fmaf(-a1, s.z, r.z));
             float v[8] = {dot3(r1, precondition(r1)), dot3(r1, r1), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            ok = reduce8<kMeet, false>(a, v, ns, red, box, epoch, &s_ok, [&](const float* T) {
+            ok = reduce8<kMeet, false>(a, team, v, ns, red, box, epoch, &s_ok, [&](const float* T) {
                 st.beta = T[0] / st.rz;
                 st.rr = T[1];
                 st.active = (st.rr > st.floor_rr) && (st.iters < a.maxiter);
@@ -646,25 +652,26 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
         }
     }
     if (threadIdx.x == 0) {
-        if (ok && blockIdx.x == 0) {
+        if (ok && blockIdx.x == (unsigned)team.x) {
             SceneStats o;
             o.iterations = st.iters;
             o.rr = st.rr;
             o.bb = st.bb;
             o.converged = st.rr <= st.floor_rr;
-            a.scene_stats[0] = o;
-            a.cum_iters[0] += st.iters;
+            a.scene_stats[team.z] = o;
+            a.cum_iters[team.z] += st.iters;
             // running max of the relative residual (non-negative floats order like their bit patterns)
             float rel = st.bb > 0.0f ? (float)sqrt(fmax((double)st.rr, 0.0) / (double)st.bb) : 0.0f;
             if (!isfinite(rel)) rel = 1.0e30f;
             atomicMax(reinterpret_cast<int*>(a.resid_max + (step_mode ? 0 : 1)), __float_as_int(rel));
         }
-        // the last CTA to leave clears the barrier for the next launch: no memset per solve
-        if (kMeet == kGrid) {
+        // the team's last CTA to leave clears its barrier for the next launch: no memset per solve
+        if (kMeet == kGrid || (kMeet == kTeams && team.y > 1)) {
             if (!ok) __threadfence();
-            if (atomicAdd(a.ticket, 1u) == gridDim.x - 1) {
-                *a.barrier = 0u;
-                *a.ticket = 0u;
+            unsigned* words = a.barrier + team.z * kTeamWords;
+            if (atomicAdd(words + kTeamTicket, 1u) == (unsigned)team.y - 1) {
+                words[0] = 0u;
+                words[kTeamTicket] = 0u;
             }
         }
     }
@@ -686,11 +693,16 @@ template <Meet kMeet>
 OcKernel oc_kernel_for(int threads, bool hybrid) {
     if (threads <= 32 * kOcWideWarps)
         return hybrid ? onchip_pcg_kernel<kOcRegs, 512, true, kMeet> : onchip_pcg_kernel<kOcRegs, 512, false, kMeet>;
-    return hybrid ? onchip_pcg_kernel<0, 1024, true, kGrid> : onchip_pcg_kernel<0, 1024, false, kGrid>;
+    constexpr Meet kWide = kMeet == kTeams ? kTeams : kGrid;
+    return hybrid ? onchip_pcg_kernel<0, 1024, true, kWide> : onchip_pcg_kernel<0, 1024, false, kWide>;
 }
 OcKernel oc_kernel(int meet, int threads, bool hybrid) {
-    return meet == kAlone ? oc_kernel_for<kAlone>(threads, hybrid)
-                          : (meet == kCluster ? oc_kernel_for<kCluster>(threads, hybrid) : oc_kernel_for<kGrid>(threads, hybrid));
+    switch (meet) {
+        case kAlone: return oc_kernel_for<kAlone>(threads, hybrid);
+        case kCluster: return oc_kernel_for<kCluster>(threads, hybrid);
+        case kGrid: return oc_kernel_for<kGrid>(threads, hybrid);
+        default: return oc_kernel_for<kTeams>(threads, hybrid);
+    }
 }
 
 cudaLaunchAttribute cluster_attribute(int ctas) {
@@ -704,11 +716,46 @@ cudaLaunchAttribute cluster_attribute(int ctas) {
 
 }  // namespace
 
+// Teams of CTAs for several scenes: the smallest number of slices per CTA that one wave holds, then the
+// CTAs left over to the scenes with the most slices per CTA.  No teams when a CTA would need more than 32.
+static void plan_teams(const Handle& h, int sms, OnchipPlan& plan) {
+    std::vector<int> s0(h.nscenes + 1, 0);
+    for (int sl = 0; sl < h.nslices; ++sl) s0[h.host_slice_scene[sl] + 1]++;
+    for (int sc = 0; sc < h.nscenes; ++sc) s0[sc + 1] += s0[sc];
+    auto slices = [&](int sc) { return s0[sc + 1] - s0[sc]; };
+    int most = std::max(1, (h.nslices + sms - 1) / sms), used = 0;
+    for (;; ++most) {
+        if (most > 32) return;
+        used = 0;
+        for (int sc = 0; sc < h.nscenes; ++sc) used += (slices(sc) + most - 1) / most;
+        if (used <= sms) break;
+    }
+    std::vector<int> ctas(h.nscenes);
+    for (int sc = 0; sc < h.nscenes; ++sc) ctas[sc] = (slices(sc) + most - 1) / most;
+    for (; used < sms; ++used) {
+        int best = -1;
+        for (int sc = 0; sc < h.nscenes; ++sc)
+            if (ctas[sc] < slices(sc) &&
+                (best < 0 || (int64_t)slices(sc) * ctas[best] > (int64_t)slices(best) * ctas[sc]))
+                best = sc;
+        if (best < 0) break;
+        ++ctas[best];
+    }
+    for (int sc = 0; sc < h.nscenes; ++sc) {
+        const int at = (int)plan.team.size();
+        for (int c = 0; c < ctas[sc]; ++c) {
+            plan.slice0.push_back(s0[sc] + (int)((int64_t)slices(sc) * c / ctas[sc]));
+            plan.team.push_back(make_int4(at, ctas[sc], sc, 0));
+        }
+    }
+    plan.slice0.push_back(h.nslices);
+}
+
 // Lays a handle out for the on-chip kernel: the CTAs' slices, their halo lists and local columns and
 // the resident share of the columns.  Leaves plan.grid 0 when the rows do not fit.
 void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& plan) {
     plan = OnchipPlan{};
-    if (h.nslices == 0 || h.nscenes != 1) return;
+    if (h.nslices == 0 || h.nscenes > sms) return;
     int width = 0;
     int64_t columns = 0;
     for (int sl = 0; sl < h.nslices; ++sl) {
@@ -719,16 +766,24 @@ void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& pl
     const int wanted = std::max(1, (width + 3) / 4);  // warps per slice: about four columns each
     int grid = std::min(sms, h.nslices);
     plan.meet = kGrid;
-    if (columns <= kAloneColumns && h.nslices <= kOcWideWarps) {
-        grid = 1;
-        plan.meet = kAlone;
-    } else if (columns <= kClusterColumns && h.nslices <= kMaxCluster * kOcWideWarps) {
-        grid = std::min(kMaxCluster, h.nslices);
-        plan.meet = kCluster;
+    if (h.nscenes > 1) {
+        plan.meet = kTeams;
+        plan_teams(h, sms, plan);
+        grid = (int)plan.team.size();
+        if (grid == 0) return;
+    } else {
+        if (columns <= kAloneColumns && h.nslices <= kOcWideWarps) {
+            grid = 1;
+            plan.meet = kAlone;
+        } else if (columns <= kClusterColumns && h.nslices <= kMaxCluster * kOcWideWarps) {
+            grid = std::min(kMaxCluster, h.nslices);
+            plan.meet = kCluster;
+        }
+        if ((h.nslices + grid - 1) / grid > (plan.meet == kGrid ? 32 : kOcWideWarps)) return;
+        // contiguous runs balanced by stored blocks
+        plan.slice0 = in.split(grid);
+        plan.team.assign(grid, make_int4(0, grid, 0, 0));
     }
-    if ((h.nslices + grid - 1) / grid > (plan.meet == kGrid ? 32 : kOcWideWarps)) return;
-    // contiguous runs balanced by stored blocks, at most 32 slices each
-    plan.slice0 = in.split(grid);
     int widest = 0;
     for (int c = 0; c < grid; ++c) widest = std::max(widest, plan.slice0[c + 1] - plan.slice0[c]);
     if (widest > 32) return;
@@ -846,6 +901,7 @@ cudaError_t launch_pcg_onchip(Handle& h, float dt, int write_state, float* q_out
     a.row_info = h.row_info;
     a.minv = h.minv;
     a.slice0 = h.oc_slice0;
+    a.team = h.oc_team;
     a.kres = h.oc_kres;
     a.halo_ptr = h.oc_halo_ptr;
     a.halo = h.oc_halo;
@@ -864,8 +920,7 @@ cudaError_t launch_pcg_onchip(Handle& h, float dt, int write_state, float* q_out
     a.rec0 = h.oc_rec0;
     a.rec1 = h.oc_rec1;
     a.part = h.oc_part;
-    a.barrier = h.barrier + kOnchipBarrier;
-    a.ticket = h.barrier + kOnchipTicket;
+    a.barrier = h.oc_barrier;
     a.status = h.status;
     a.scene_stats = h.scene_stats;
     a.cum_iters = h.cum_iters;

@@ -249,3 +249,22 @@ def test_onchip_kernel_solves_the_streaming_kernels_system(element, cells):
     for a, b, c in zip(got, again, ref):
         np.testing.assert_array_equal(a, b)
         assert rel_l2(a, c) < 1e-5
+
+
+@pytest.mark.parametrize("count,dims", [(2, (2, 3)), (24, (3, 10)), (9, (2, 24)), (152, (2, 5))],
+                         ids=lambda v: str(v).replace(" ", ""))
+def test_onchip_teams_solve_the_streaming_kernels_batch(count, dims):
+    """Scenes of one to many slices as teams of one to many CTAs, up to a scene per SM: the launch
+    variants' bound against the streaming kernel, and repeated substeps are bit-identical."""
+    sc = scenes.batched_scenes(count=count, seed=7, dims=dims)
+    model, solver, _ = scene_pair(sc, linear_solver_tolerance=1e-6, linear_solver_maxiter=200, with_oracle=False)
+    lib = _lib.load()
+    assert setting(solver, _lib.FEM_TUNE_ONCHIP_GRID) >= count
+    got, again = substep(model, solver, sc), substep(model, solver, sc)
+    its = solver.stats()["scene_iterations"]
+    _lib.check(lib.fem_set_tuning(solver._handle, _lib.FEM_TUNE_ONCHIP, 0))
+    ref = substep(model, solver, sc)
+    assert max(abs(a - b) for a, b in zip(its, solver.stats()["scene_iterations"])) <= 1
+    for a, b, c in zip(got, again, ref):
+        np.testing.assert_array_equal(a, b)
+        assert rel_l2(a, c) < 1e-5
