@@ -721,9 +721,7 @@ cudaError_t launch_predictor_vjp(Handle& h, const float* rhs_bar, float dt, floa
 cudaError_t rollout_substep(Handle& h, float* q_in, float* v_in, float* q_out, float* v_out, const float* ext,
                             const float* act, const float* gravity, float dt, float tol, int maxiter, bool warm,
                             cudaStream_t s) {
-    cudaError_t err = cudaSuccess;
-    if (!warm) err = cudaMemsetAsync(h.dv, 0, sizeof(float) * 3 * (size_t)h.P, s);
-    if (err == cudaSuccess) err = fem::launch_node_prepare(h, q_in, v_in, true, true, true, s);
+    cudaError_t err = fem::launch_node_prepare(h, q_in, v_in, true, true, true, s, /*zero_x=*/!warm);
     if (err == cudaSuccess) err = fem::launch_element_forces(h, act, s);
     if (err == cudaSuccess) err = fem::launch_node_forces(h, ext, gravity, dt, FEM_TERM_ALL, true, h.roll_f, s);
     if (err == cudaSuccess) err = fem::launch_pcg(h, dt, 1, q_out, v_out, h.roll_f, s, nullptr, nullptr, tol, maxiter);

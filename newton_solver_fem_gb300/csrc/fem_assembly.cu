@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(256, 6) gather_kernel(int64_t nsell, int P, co
                               const unsigned* __restrict__ contrib,
                               const TripletPlanes trip, float4* __restrict__ valA, float4* __restrict__ valB,
                               float* __restrict__ valC, float* __restrict__ minv, int precond, int clear_empty) {
+    chained_start();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nsell) return;
     const int c0 = cptr[e], c1 = cptr[e + 1];
@@ -157,9 +158,9 @@ cudaError_t launch_gather(Handle& h, cudaStream_t s) {
     if (h.nsell == 0) return cudaSuccess;
     int threads = 256;
     int64_t blocks = (h.nsell + threads - 1) / threads;
-    gather_kernel<<<(unsigned)blocks, threads, 0, s>>>(h.nsell, h.P, h.sell_cptr,
-                                                       reinterpret_cast<const unsigned*>(h.sell_contrib), h.trip, h.valA,
-                                                       h.valB, h.valC, h.minv, h.precond, h.streaming);
+    launch_maybe_chained(blocks <= kChainedBlocks, gather_kernel, (unsigned)blocks, threads, 0, s, h.nsell, h.P,
+                         h.sell_cptr, reinterpret_cast<const unsigned*>(h.sell_contrib), h.trip, h.valA, h.valB, h.valC,
+                         h.minv, h.precond, h.streaming);
     return cudaGetLastError();
 }
 

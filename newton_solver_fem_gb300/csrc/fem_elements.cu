@@ -33,13 +33,14 @@ __global__ void node_prepare_kernel(int P, float* __restrict__ q, float* __restr
                                     const unsigned char* __restrict__ fixed_mask, const float* __restrict__ rest,
                                     const float* __restrict__ dv, float4* __restrict__ q4, float4* __restrict__ v4,
                                     float4* __restrict__ x4, int restore, int pack_v, int pack_x) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
     bool fx = fixed_mask[i] != 0;
     if (!restore) {  // plain packing, caller arrays untouched
         q4[i] = f4(load3(q, i));
         if (pack_v) v4[i] = f4(load3(v, i));
-        if (pack_x) x4[i] = fx ? make_float4(0.f, 0.f, 0.f, 0.f) : f4(load3(dv, i));
+        if (pack_x) x4[i] = (fx || pack_x == 2) ? make_float4(0.f, 0.f, 0.f, 0.f) : f4(load3(dv, i));
         return;
     }
     float3 qi;
@@ -56,7 +57,7 @@ __global__ void node_prepare_kernel(int P, float* __restrict__ q, float* __restr
         else vi = load3(v, i);
         v4[i] = f4(vi);
     }
-    if (pack_x) x4[i] = fx ? make_float4(0.f, 0.f, 0.f, 0.f) : f4(load3(dv, i));
+    if (pack_x) x4[i] = (fx || pack_x == 2) ? make_float4(0.f, 0.f, 0.f, 0.f) : f4(load3(dv, i));
 }
 
 // Reference kernels.py:511-632 (force) and 484-508 (activation).  Writes the
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(128, 8) tet_force_kernel(int T, const int4* __
                                  const float* __restrict__ mat, const float4* __restrict__ q4,
                                  const float4* __restrict__ v4, const float* __restrict__ act,
                                  const float* __restrict__ mu_scale, float lo, float hi, float4* __restrict__ out) {
+    chained_start();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
     int4 n = idx[t];
@@ -156,6 +158,7 @@ __global__ void __launch_bounds__(256, 4) hex_force_kernel(int H, const int* __r
                                                         const float4* __restrict__ q4,
                                                         const float4* __restrict__ v4, float lo, float hi,
                                                         float4* __restrict__ out) {
+    chained_start();
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     const int h = gid >> 3, g = gid & 7;
     const bool live = h < H;
@@ -245,6 +248,7 @@ __global__ void __launch_bounds__(256, 4) hex_force_kernel(int H, const int* __r
 __global__ void tri_force_kernel(int Tri, const int* __restrict__ idx, const float4* __restrict__ pose,
                                  const float* __restrict__ mat, const float4* __restrict__ q4,
                                  const float4* __restrict__ v4, float4* __restrict__ out) {
+    chained_start();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= Tri) return;
     V3<float> x[3], v[3], f[3];
@@ -308,6 +312,7 @@ struct NodeForceArgs {
 // none: the remaining gather then fits in fewer registers, so more warps cover its load latency.
 template <bool kFull>
 __global__ void node_forces_kernel(NodeForceArgs a) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.P) return;
     float3 xi = xyz(a.q4[i]), vi = xyz(a.v4[i]);
@@ -511,6 +516,7 @@ __global__ void __launch_bounds__(kTetTangentThreads) tet_tangent_kernel(
     int T, const int4* __restrict__ idx, const float* __restrict__ pose, const float* __restrict__ mat,
     const float* __restrict__ mu_scale, const float4* __restrict__ q4, float lo, float hi, float dt, int64_t trip_off,
     TripletPlanes vals) {
+    chained_start();
     __shared__ float sm[kTetTangentThreads][kTetFactor + 1];
     int lt = threadIdx.x;
     int t = blockIdx.x * kTetTangentThreads + lt;
@@ -732,6 +738,7 @@ __global__ void __launch_bounds__(kTanThreads, 4) hex_tangent_kernel(int H, cons
                                                                       const float4* __restrict__ q4, float lo,
                                                                       float hi, float dt, int64_t trip_off,
                                                                       TripletPlanes vals) {
+    chained_start();
     extern __shared__ __align__(16) unsigned char smem[];
     float* s_rec = reinterpret_cast<float*>(smem);
     float4* s_x = reinterpret_cast<float4*>(smem + kTanXOff);     // [hex][node]
@@ -895,27 +902,27 @@ void fill_hex_reference_table(float table[8][8][3]) {
 }
 
 cudaError_t launch_node_prepare(Handle& h, float* q, float* v, bool restore_fixed, bool pack_v, bool pack_x,
-                                cudaStream_t s) {
+                                cudaStream_t s, bool zero_x) {
     if (h.P == 0) return cudaSuccess;
-    node_prepare_kernel<<<blocks_for(h.P, 256), 256, 0, s>>>(h.P, q, v, h.fixed_mask, h.rest, h.dv, h.q4, h.v4, h.x,
-                                                             restore_fixed ? 1 : 0, pack_v ? 1 : 0, pack_x ? 1 : 0);
+    launch_chained(node_prepare_kernel, blocks_for(h.P, 256), 256, 0, s, h.P, q, v, h.fixed_mask, h.rest, h.dv, h.q4,
+                   h.v4, h.x, restore_fixed ? 1 : 0, pack_v ? 1 : 0, pack_x ? (zero_x ? 2 : 1) : 0);
     return cudaGetLastError();
 }
 
 cudaError_t launch_element_forces(Handle& h, const float* activations, cudaStream_t s) {
     if (h.T > 0) {
-        tet_force_kernel<<<blocks_for(h.T, 128), 128, 0, s>>>(h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.q4, h.v4,
-                                                              h.enable_act ? activations : nullptr, h.mu_scale,
-                                                              h.min_stretch, h.max_stretch, h.elem_force);
+        launch_chained(tet_force_kernel, blocks_for(h.T, 128), 128, 0, s, h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.q4,
+                       h.v4, h.enable_act ? activations : nullptr, h.mu_scale, h.min_stretch, h.max_stretch,
+                       h.elem_force);
     }
     if (h.H > 0) {
-        hex_force_kernel<<<blocks_for(8 * (int64_t)h.H, 256), 256, 0, s>>>(
-            h.H, h.hex_idx, h.hex_invJ, h.hex_detw, h.hex_mat, h.q4, h.v4, h.min_stretch, h.max_stretch,
-            h.elem_force + 4 * (int64_t)h.T);
+        launch_chained(hex_force_kernel, blocks_for(8 * (int64_t)h.H, 256), 256, 0, s, h.H, h.hex_idx, h.hex_invJ,
+                       h.hex_detw, h.hex_mat, h.q4, h.v4, h.min_stretch, h.max_stretch,
+                       h.elem_force + 4 * (int64_t)h.T);
     }
     if (h.Tri > 0)
-        tri_force_kernel<<<blocks_for(h.Tri, 128), 128, 0, s>>>(h.Tri, h.tri_idx, h.tri_pose, h.tri_mat, h.q4, h.v4,
-                                                                h.elem_force + 4 * (int64_t)h.T + 8 * (int64_t)h.H);
+        launch_chained(tri_force_kernel, blocks_for(h.Tri, 128), 128, 0, s, h.Tri, h.tri_idx, h.tri_pose, h.tri_mat,
+                       h.q4, h.v4, h.elem_force + 4 * (int64_t)h.T + 8 * (int64_t)h.H);
     return cudaGetLastError();
 }
 
@@ -981,8 +988,8 @@ cudaError_t launch_node_forces(Handle& h, const float* ext, const float* gravity
     a.out = out;
     const bool full = (h.S > 0 && (terms & FEM_TERM_SPRING)) || a.pforce != nullptr || a.sc_head != nullptr ||
                       a.sforce != nullptr;
-    if (full) node_forces_kernel<true><<<blocks_for(h.P, 128), 128, 0, s>>>(a);
-    else node_forces_kernel<false><<<blocks_for(h.P, 128), 128, 0, s>>>(a);
+    if (full) launch_chained(node_forces_kernel<true>, blocks_for(h.P, 128), 128, 0, s, a);
+    else launch_chained(node_forces_kernel<false>, blocks_for(h.P, 128), 128, 0, s, a);
     return cudaGetLastError();
 }
 
@@ -1002,14 +1009,16 @@ cudaError_t launch_constant_blocks(Handle& h, float dt, cudaStream_t s) {
 cudaError_t launch_element_tangent(Handle& h, float dt, cudaStream_t s) {
     int64_t tet_off = tet_triplet_offset(h);
     if (h.T > 0)
-        tet_tangent_kernel<<<blocks_for(h.T, kTetTangentThreads), kTetTangentThreads, 0, s>>>(
-            h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.mu_scale, h.q4, h.min_stretch, h.max_stretch, dt, tet_off,
+        launch_maybe_chained(
+            blocks_for(h.T, kTetTangentThreads) <= (int)kChainedBlocks, tet_tangent_kernel,
+            blocks_for(h.T, kTetTangentThreads), kTetTangentThreads, 0, s, h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.mu_scale, h.q4, h.min_stretch, h.max_stretch, dt, tet_off,
             h.trip);
     if (h.H > 0) {
         cudaError_t err = allow_dynamic_smem((const void*)hex_tangent_kernel, kTanSmemBytes);
         if (err != cudaSuccess) return err;
-        hex_tangent_kernel<<<blocks_for(h.H, kTanHex), kTanThreads, kTanSmemBytes, s>>>(
-            h.H, h.hex_idx, h.hex_invJ, h.hex_detw, h.hex_mat, h.q4, h.min_stretch, h.max_stretch, dt,
+        launch_maybe_chained(
+            blocks_for(h.H, kTanHex) <= (int)kChainedBlocks, hex_tangent_kernel, blocks_for(h.H, kTanHex), kTanThreads,
+            kTanSmemBytes, s, h.H, h.hex_idx, h.hex_invJ, h.hex_detw, h.hex_mat, h.q4, h.min_stretch, h.max_stretch, dt,
             h.trip_map.hex_start(), h.trip);
     }
     return cudaGetLastError();

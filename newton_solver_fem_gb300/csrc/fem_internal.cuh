@@ -70,6 +70,41 @@ __device__ __forceinline__ void store_block(const TripletPlanes& t, int64_t i, c
 }
 #endif
 
+// Kernels that follow one another on a stream are launched as programmatic dependents: a kernel lets its
+// successor be launched as soon as all of its own CTAs run, and the successor's CTAs wait, before they
+// touch memory, until every kernel before them has completed and its writes are visible.  The order is
+// the stream's, as before; what goes is the launch latency between two short kernels (eagerly and in
+// captured graphs): a substep's five launches take 10 us less.  A kernel launched this way begins with
+// chained_start().  The tangent and the assembly are chained only while their grid is at most
+// kChainedBlocks: a 1,500-CTA assembly behind an early start, with device copies after it, made the
+// refresh and export of 26,220 Tet4 nodes 125 us instead of 84 (and 48^3 Hex8 251 instead of 230).
+#ifdef __CUDACC__
+__device__ __forceinline__ void chained_start() {
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+#endif
+constexpr unsigned kChainedBlocks = 304;
+template <class... Params, class... Args>
+inline cudaError_t launch_maybe_chained(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                        cudaStream_t s, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                  Args&&... args) {
+    return launch_maybe_chained(true, kernel, grid, block, smem, s, args...);
+}
+
 // Per-scene persistent solver statistics written by the PCG epilogue.
 struct SceneStats {
     int iterations;
@@ -383,8 +418,9 @@ void upload_hex_reference_table();          // fem_elements.cu copy
 void upload_hex_reference_table_adjoint();  // fem_adjoint.cu copy
 
 // --- launchers (fem_elements.cu) ---
+// zero_x: with pack_x, a zero warm start instead of dv
 cudaError_t launch_node_prepare(Handle& h, float* q, float* v, bool restore_fixed, bool pack_v, bool pack_x,
-                                cudaStream_t s);
+                                cudaStream_t s, bool zero_x = false);
 cudaError_t launch_element_forces(Handle& h, const float* activations, cudaStream_t s);
 cudaError_t launch_node_forces(Handle& h, const float* ext, const float* gravity, float dt, int terms, bool scale_by_dt,
                                float* out, cudaStream_t s);

@@ -338,6 +338,7 @@ __device__ __forceinline__ bool reduce8(const OcArgs& a, int4 team, float (&v)[8
 
 template <int kRegs, int kThreads, bool kHybrid, Meet kMeet>
 __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
+    chained_start();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ OcState st;
     __shared__ int s_ok;
@@ -937,15 +938,17 @@ cudaError_t launch_pcg_onchip(Handle& h, float dt, int write_state, float* q_out
     cfg.blockDim = dim3(h.oc_threads);
     cfg.dynamicSmemBytes = h.oc_smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     if (h.oc_meet == kCluster) {
-        attr[0] = cluster_attribute(h.oc_grid);
+        attr[1] = cluster_attribute(h.oc_grid);
     } else {
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
+        attr[1].id = cudaLaunchAttributeCooperative;
+        attr[1].val.cooperative = 1;
     }
     cfg.attrs = attr;
-    cfg.numAttrs = h.oc_meet == kAlone ? 0 : 1;  // one CTA waits for no other
+    cfg.numAttrs = h.oc_meet == kAlone ? 1 : 2;  // one CTA waits for no other
     return cudaLaunchKernelEx(&cfg, oc_kernel(h.oc_meet, h.oc_threads, h.oc_hybrid != 0), a);
 }
 

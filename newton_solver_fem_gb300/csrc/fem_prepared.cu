@@ -37,6 +37,7 @@ __global__ void prepare_state_kernel(int P, const float* __restrict__ q_in, cons
                                      const unsigned char* __restrict__ fixed, const float* __restrict__ rest,
                                      float* __restrict__ pq, float* __restrict__ pv, float4* __restrict__ q4,
                                      float4* __restrict__ v4) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
     const bool fx = fixed[i] != 0;
@@ -55,6 +56,7 @@ __global__ void predictor_diag_kernel(int nslices, const int* __restrict__ slice
                                       const float4* __restrict__ valB, const float* __restrict__ valC,
                                       const int* __restrict__ scol, const float4* __restrict__ v4,
                                       float* __restrict__ pred, float* __restrict__ diag) {
+    chained_start();
     const int sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (sl >= nslices) return;
     const int2 m = meta[sl];
@@ -90,6 +92,7 @@ __global__ void prepared_rhs_kernel(int P, const float* __restrict__ impulse, co
                                     const int* __restrict__ sent, const int* __restrict__ sidx,
                                     const float* __restrict__ skd, const float* __restrict__ pv,
                                     const unsigned char* __restrict__ fixed, float* __restrict__ out) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
     if (fixed[i]) {
@@ -328,6 +331,7 @@ __global__ void apply_preconditioner_kernel(int P, const float* __restrict__ min
 
 __global__ void pack_warm_start_kernel(int P, const float* __restrict__ dv, const unsigned char* __restrict__ fixed,
                                        float4* __restrict__ x4) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
     x4[i] = fixed[i] ? make_float4(0.f, 0.f, 0.f, 0.f) : f4(ld3(dv, i));
@@ -338,6 +342,7 @@ __global__ void reconstruct_kernel(int P, const float* __restrict__ dv, const fl
                                    const float* __restrict__ pv, const unsigned char* __restrict__ fixed,
                                    const float* __restrict__ rest, float dt, float* __restrict__ q_out,
                                    float* __restrict__ v_out) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
     float3 v = ld3(pv, i) + ld3(dv, i);
@@ -370,9 +375,8 @@ struct Guard {
 
 
 cudaError_t launch_rhs(Handle& h, const FemPreparedWs* w, const float* ext, float dt, float* out, cudaStream_t s) {
-    prepared_rhs_kernel<<<blocks(h.P, 256), 256, 0, s>>>(h.P, w->impulse, ext, dt, w->predictor, h.node_spring_ptr,
-                                                         h.node_spring_ent, h.spring_idx, h.spring_kd, w->v,
-                                                         h.fixed_mask, out);
+    launch_chained(prepared_rhs_kernel, blocks(h.P, 256), 256, 0, s, h.P, w->impulse, ext, dt, w->predictor,
+                   h.node_spring_ptr, h.node_spring_ent, h.spring_idx, h.spring_kd, w->v, h.fixed_mask, out);
     return cudaGetLastError();
 }
 
@@ -395,16 +399,16 @@ int fem_prepare(FemHandle* H, const FemPreparedWs* w, const float* q_in, const f
     if (h.P == 0) return FEM_OK;
     fem::Guard g(H->device);
     cudaStream_t s = (cudaStream_t)stream;
-    fem::prepare_state_kernel<<<fem::blocks(h.P, 256), 256, 0, s>>>(h.P, q_in, v_in, h.fixed_mask, h.rest, w->q,
-                                                                      w->v, h.q4, h.v4);
+    fem::launch_chained(fem::prepare_state_kernel, fem::blocks(h.P, 256), 256, 0, s, h.P, q_in, v_in, h.fixed_mask,
+                        h.rest, w->q, w->v, h.q4, h.v4);
     cudaError_t err = cudaGetLastError();
     if (err == cudaSuccess) err = fem::launch_element_forces(h, activations, s);
     if (err == cudaSuccess)
         err = fem::launch_node_forces(h, external_forces, gravity, dt, FEM_TERM_ALL, true, w->impulse, s);
     if (err == cudaSuccess && h.nslices > 0) {
-        fem::predictor_diag_kernel<<<fem::blocks((int64_t)h.nslices * 32, 256), 256, 0, s>>>(
-            h.nslices, h.slice_ptr, h.slice_meta, h.row_info, h.valA, h.valB, h.valC, h.scol, h.v4, w->predictor,
-            w->diagonal);
+        fem::launch_chained(fem::predictor_diag_kernel, fem::blocks((int64_t)h.nslices * 32, 256), 256, 0, s, h.nslices,
+                            h.slice_ptr, h.slice_meta, h.row_info, h.valA, h.valB, h.valC, h.scol, h.v4, w->predictor,
+                            w->diagonal);
         err = cudaGetLastError();
     }
     if (err == cudaSuccess) err = fem::launch_rhs(h, w, nullptr, dt, w->base_rhs, s);
@@ -476,7 +480,7 @@ int fem_prepared_solve(FemHandle* H, const FemPreparedWs* w, const float* rhs, f
     if (h.P == 0) return FEM_OK;
     fem::Guard g(H->device);
     cudaStream_t s = (cudaStream_t)stream;
-    fem::pack_warm_start_kernel<<<fem::blocks(h.P, 256), 256, 0, s>>>(h.P, w->increment, h.fixed_mask, h.x);
+    fem::launch_chained(fem::pack_warm_start_kernel, fem::blocks(h.P, 256), 256, 0, s, h.P, w->increment, h.fixed_mask, h.x);
     cudaError_t err = cudaGetLastError();
     if (err == cudaSuccess)
         err = fem::launch_pcg(h, dt, 0, nullptr, nullptr, nullptr, s, rhs, w->increment, tolerance, maxiter,
@@ -493,8 +497,7 @@ int fem_prepared_reconstruct(FemHandle* H, const FemPreparedWs* w, const float* 
     Handle& h = H->h;
     if (h.P == 0) return FEM_OK;
     fem::Guard g(H->device);
-    fem::reconstruct_kernel<<<fem::blocks(h.P, 256), 256, 0, (cudaStream_t)stream>>>(
-        h.P, dv, w->q, w->v, h.fixed_mask, h.rest, dt, q_out, v_out);
+    fem::launch_chained(fem::reconstruct_kernel, fem::blocks(h.P, 256), 256, 0, (cudaStream_t)stream, h.P, dv, w->q, w->v, h.fixed_mask, h.rest, dt, q_out, v_out);
     return fem::report_cuda(cudaGetLastError());
 }
 
