@@ -134,33 +134,23 @@ class _Substep(torch.autograd.Function):
         has_ext, has_act, has_scale = ctx.has
         dt = ctx.dt
         lib = diff.lib
-        handle = diff.solver._handle
-        stream = diff._stream()
-        qb = torch.zeros_like(q_in) if q_out_bar is None else q_out_bar.contiguous().clone()
-        vb = torch.zeros_like(v_in) if v_out_bar is None else v_out_bar.contiguous().clone()
-        qb[diff.fixed] = 0.0  # fixed outputs are overwritten by the restore
-        vb[diff.fixed] = 0.0
-        vt = torch.add(vb, qb, alpha=dt)  # one rounding, as the device schedule's seed kernel
-        rhs_bar = diff.solve(vt)
-        if diff.after_backward_solve is not None:
-            diff.after_backward_solve()
-        v_bar = vt.clone()
-        _lib.check(lib.fem_predictor_vjp(handle, rhs_bar.data_ptr(), dt, v_bar.data_ptr(), stream))
-        q_bar = qb
-        g = (dt * rhs_bar).contiguous()
+        # the whole reverse substep in one call: seed (outputs at fixed nodes carry no gradient), adjoint
+        # solve, predictor and force VJPs, fixed inputs zeroed; it updates q_bar and v_bar in place
+        q_bar = torch.zeros_like(q_in) if q_out_bar is None else q_out_bar.contiguous().clone()
+        v_bar = torch.zeros_like(v_in) if v_out_bar is None else v_out_bar.contiguous().clone()
         T = diff.model.tet_count
+        ext_bar = torch.zeros_like(q_in) if has_ext else None
         act_bar = torch.zeros(T, dtype=torch.float32, device=q_in.device) if has_act else None
         scale_bar = torch.zeros(T, dtype=torch.float32, device=q_in.device) if has_scale else None
         if has_scale:
             diff.set_mu_scale(scale)
-        _lib.check(lib.fem_force_vjp(handle, q_in.data_ptr(), v_in.data_ptr(),
-                                     act.data_ptr() if has_act else None, diff.model.gravity.data_ptr(), g.data_ptr(),
-                                     q_bar.data_ptr(), v_bar.data_ptr(),
-                                     act_bar.data_ptr() if has_act else None,
-                                     scale_bar.data_ptr() if has_scale else None, stream), "force VJP")
-        q_bar[diff.fixed] = 0.0  # fixed inputs are overwritten by the restore
-        v_bar[diff.fixed] = 0.0
-        ext_bar = g if has_ext else None
+        ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+        _lib.check(lib.fem_adjoint_segment(
+            diff.solver._handle, q_in.data_ptr(), v_in.data_ptr(), 1, None, act.data_ptr() if has_act else None,
+            diff.model.gravity.data_ptr(), dt, diff.tolerance, diff.maxiter, 0, None, q_bar.data_ptr(),
+            v_bar.data_ptr(), ptr(ext_bar), ptr(act_bar), ptr(scale_bar), None, None, diff._stream()), "adjoint substep")
+        if diff.after_backward_solve is not None:
+            diff.after_backward_solve()
         return None, q_bar, v_bar, None, ext_bar, act_bar, scale_bar
 
 

@@ -25,20 +25,6 @@
 
 namespace fem {
 namespace {
-__constant__ float c_dNdxi[8][8][3];  // this translation unit's copy of the Gauss table
-}  // namespace
-
-void upload_hex_reference_table_adjoint() {
-    static bool done[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-    if (done[dev]) return;
-    float table[8][8][3];
-    fill_hex_reference_table(table);
-    if (cudaMemcpyToSymbol(c_dNdxi, table, sizeof(table)) == cudaSuccess) done[dev] = true;
-}
-
-namespace {
 
 __device__ __forceinline__ float3 ld3(const float* p, int i) { return f3(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
 __device__ __forceinline__ void add3(float* p, int i, float3 v) {
@@ -69,6 +55,7 @@ __global__ void tet_force_vjp_kernel(int T, const int4* __restrict__ idx, const 
                                      const float* __restrict__ act, const float* __restrict__ g, float gs, float lo,
                                      float hi, float4* __restrict__ grad, float* __restrict__ act_bar,
                                      float* __restrict__ scale_bar, float* __restrict__ mat_bar, int acc) {
+    chained_start();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
     float4* o = grad + 8 * (size_t)t;  // [corner][x-bar, v-bar]
@@ -210,6 +197,7 @@ __global__ void hex_force_vjp_kernel(int H, const int* __restrict__ idx, const f
                                      const float4* __restrict__ q4, const float4* __restrict__ v4,
                                      const float* __restrict__ g, float gs, float lo, float hi,
                                      float4* __restrict__ grad, float* __restrict__ mat_bar, int acc) {
+    chained_start();
     int gid = blockIdx.x * blockDim.x + threadIdx.x;
     int h = gid >> 3, gp = gid & 7;
     bool live = h < H;
@@ -223,6 +211,9 @@ __global__ void hex_force_vjp_kernel(int H, const int* __restrict__ idx, const f
     for (int k = 0; k < 9; ++k) iJ.m[k / 3][k % 3] = invJ[(8 * he + gp) * 9 + k];
     float w = detw[8 * he + gp];
     int base = threadIdx.x & 24;
+    const float gauss = 0.5773502691896258f;
+    const float xi = ((gp ^ (gp >> 1)) & 1) ? gauss : -gauss, eta = (gp & 2) ? gauss : -gauss,
+                zeta = (gp & 4) ? gauss : -gauss;
     float3 dN[8], gb[8];
     M3 F, dF;
 #pragma unroll
@@ -237,7 +228,11 @@ __global__ void hex_force_vjp_kernel(int H, const int* __restrict__ idx, const f
                        __shfl_sync(0xffffffffu, vg.z, base + a));
         gb[a] = f3(__shfl_sync(0xffffffffu, gg.x, base + a), __shfl_sync(0xffffffffu, gg.y, base + a),
                    __shfl_sync(0xffffffffu, gg.z, base + a));
-        dN[a] = mulT(iJ, f3(c_dNdxi[gp][a][0], c_dNdxi[gp][a][1], c_dNdxi[gp][a][2]));
+        // dN_a/dxi at this lane's point, the reference table's own products (a constant table indexed by the
+        // lane's point is read once per distinct point)
+        const float xa1 = ((a ^ (a >> 1)) & 1) ? 1.0f : -1.0f, ya1 = (a & 2) ? 1.0f : -1.0f, za1 = (a & 4) ? 1.0f : -1.0f;
+        const float fx = 1.0f + xa1 * xi, fy = 1.0f + ya1 * eta, fz = 1.0f + za1 * zeta;
+        dN[a] = mulT(iJ, f3(xa1 * fy * fz * 0.125f, fx * ya1 * fz * 0.125f, fx * fy * za1 * 0.125f));
         float xs[3] = {xa.x, xa.y, xa.z}, vs[3] = {va.x, va.y, va.z};
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -318,24 +313,34 @@ __global__ void hex_force_vjp_kernel(int H, const int* __restrict__ idx, const f
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) Fb.m[i][j] += 2.0f * Icb * F.m[i][j] + Jb * cof.m[i][j] + cb3.m[i][j];
-    float3 xm = f3(0.f, 0.f, 0.f), vm = f3(0.f, 0.f, 0.f);
+    // Sums over the points, node by node, lane a keeping node a: each exchange halves the nodes a lane
+    // carries (42 shuffles; a butterfly per node takes 144).  The association is the butterfly's.
+    auto keep = [&](const float (&even)[6], const float (&odd)[6], float (&out)[6], int bit) {
+        const bool hi = gp & bit;
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-        float3 xa = mul(Fb, dN[a]), va = mul(dFb, dN[a]);
+        for (int k = 0; k < 6; ++k)
+            out[k] = (hi ? odd[k] : even[k]) + __shfl_xor_sync(0xffffffffu, hi ? even[k] : odd[k], bit);
+    };
+    auto corner = [&](int a, float (&o)[6]) {
+        const float3 xa = mul(Fb, dN[a]), va = mul(dFb, dN[a]);
+        o[0] = xa.x; o[1] = xa.y; o[2] = xa.z;
+        o[3] = va.x; o[4] = va.y; o[5] = va.z;
+    };
+    float quarter[2][6], own[6];
 #pragma unroll
-        for (int off = 1; off < 8; off <<= 1) {
-            xa.x += __shfl_xor_sync(0xffffffffu, xa.x, off);
-            xa.y += __shfl_xor_sync(0xffffffffu, xa.y, off);
-            xa.z += __shfl_xor_sync(0xffffffffu, xa.z, off);
-            va.x += __shfl_xor_sync(0xffffffffu, va.x, off);
-            va.y += __shfl_xor_sync(0xffffffffu, va.y, off);
-            va.z += __shfl_xor_sync(0xffffffffu, va.z, off);
+    for (int m = 0; m < 2; ++m) {
+        float pair[2][6];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            float e[6], o[6];
+            corner(4 * m + 2 * n, e);
+            corner(4 * m + 2 * n + 1, o);
+            keep(e, o, pair[n], 1);
         }
-        if (a == gp) {
-            xm = xa;
-            vm = va;
-        }
+        keep(pair[0], pair[1], quarter[m], 2);
     }
+    keep(quarter[0], quarter[1], own, 4);
+    const float3 xm = f3(own[0], own[1], own[2]), vm = f3(own[3], own[4], own[5]);
     if (live) {
         grad[2 * (8 * (size_t)h + gp)] = f4(xm);
         grad[2 * (8 * (size_t)h + gp) + 1] = f4(vm);
@@ -355,6 +360,7 @@ __global__ void tri_force_vjp_kernel(int Tri, const int* __restrict__ idx, const
                                      const float* __restrict__ mat, const float4* __restrict__ q4,
                                      const float4* __restrict__ v4, const float* __restrict__ g, float gs,
                                      float4* __restrict__ grad) {
+    chained_start();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= Tri) return;
     int n[3];
@@ -438,13 +444,29 @@ struct NodeVjpArgs {
 };
 
 __global__ void node_vjp_kernel(NodeVjpArgs a) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.P) return;
     float3 xb = f3(0.f, 0.f, 0.f), vb = f3(0.f, 0.f, 0.f);
-    for (int e = a.elem_ptr[i]; e < a.elem_ptr[i + 1]; ++e) {
-        int ent = a.elem_ent[e];
-        xb = xb + xyz(a.elem_grad[2 * (size_t)ent]);
-        vb = vb + xyz(a.elem_grad[2 * (size_t)ent + 1]);
+    // corners read kCornerBatch at a time before any is added, in ascending incidence order
+    constexpr int kCornerBatch = 4;
+    const int e1 = a.elem_ptr[i + 1];
+    for (int e0 = a.elem_ptr[i]; e0 < e1; e0 += kCornerBatch) {
+        int ent[kCornerBatch];
+        float4 x[kCornerBatch], v[kCornerBatch];
+#pragma unroll
+        for (int u = 0; u < kCornerBatch; ++u) ent[u] = __ldg(a.elem_ent + min(e0 + u, e1 - 1));
+#pragma unroll
+        for (int u = 0; u < kCornerBatch; ++u) {
+            x[u] = a.elem_grad[2 * (size_t)ent[u]];
+            v[u] = a.elem_grad[2 * (size_t)ent[u] + 1];
+        }
+#pragma unroll
+        for (int u = 0; u < kCornerBatch; ++u)
+            if (e0 + u < e1) {
+                xb = xb + xyz(x[u]);
+                vb = vb + xyz(v[u]);
+            }
     }
     for (int e = a.spring_ptr[i]; e < a.spring_ptr[i + 1]; ++e) {
         int ent = a.spring_ent[e];
@@ -530,6 +552,7 @@ __global__ void node_vjp_kernel(NodeVjpArgs a) {
 // keeps q'-bar (q' = q + h v').
 __global__ void adjoint_seed_kernel(int P, float h, const unsigned char* __restrict__ fixed, float* __restrict__ q_bar,
                                     float* __restrict__ v_bar, float* __restrict__ vt) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
     const bool fx = fixed[i] != 0;
@@ -547,6 +570,7 @@ __global__ void adjoint_seed_kernel(int P, float h, const unsigned char* __restr
 
 __global__ void pack_adjoint_start_kernel(int P, const float* __restrict__ x, const unsigned char* __restrict__ fixed,
                                           float4* __restrict__ x4) {
+    chained_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
     x4[i] = fixed[i] ? make_float4(0.f, 0.f, 0.f, 0.f) : f4(ld3(x, i));
@@ -560,6 +584,7 @@ __global__ void predictor_vjp_kernel(int nslices, const int* __restrict__ slice_
                                      const int* __restrict__ sptr, const int* __restrict__ sent,
                                      const int* __restrict__ sidx, const float* __restrict__ skd, float dt,
                                      float* __restrict__ v_bar) {
+    chained_start();
     int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (warp_global >= nslices) return;
@@ -570,15 +595,32 @@ __global__ void predictor_vjp_kernel(int nslices, const int* __restrict__ slice_
     int base = slice_ptr[warp_global];
     float3 ar = f3(0.f, 0.f, 0.f);
     float R[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int k = 0; k < len; ++k) {
-        size_t e = (size_t)(base + k) * kSlice + lane;
-        float4 A = valA[e], B = valB[e];
-        float C = valC[e];
-        float3 p = ld3(rb, scol[e]);
-        ar = ar + f3(A.x * p.x + A.y * p.y + A.z * p.z, A.w * p.x + B.x * p.y + B.y * p.z,
-                     B.z * p.x + B.w * p.y + C * p.z);
-        R[0] += A.x; R[1] += A.y; R[2] += A.z; R[3] += A.w; R[4] += B.x;
-        R[5] += B.y; R[6] += B.z; R[7] += B.w; R[8] += C;
+    // kColumnBatch blocks (and then their columns' values) in flight before any is used
+    constexpr int kColumnBatch = 4;
+    for (int k0 = 0; k0 < len; k0 += kColumnBatch) {
+        float4 A[kColumnBatch], B[kColumnBatch];
+        float C[kColumnBatch];
+        int j[kColumnBatch];
+#pragma unroll
+        for (int u = 0; u < kColumnBatch; ++u) {
+            const size_t e = (size_t)(base + min(k0 + u, len - 1)) * kSlice + lane;
+            A[u] = valA[e];
+            B[u] = valB[e];
+            C[u] = valC[e];
+            j[u] = scol[e];
+        }
+        float3 p[kColumnBatch];
+#pragma unroll
+        for (int u = 0; u < kColumnBatch; ++u) p[u] = ld3(rb, j[u]);
+#pragma unroll
+        for (int u = 0; u < kColumnBatch; ++u)
+            if (k0 + u < len) {
+                ar = ar + f3(A[u].x * p[u].x + A[u].y * p[u].y + A[u].z * p[u].z,
+                             A[u].w * p[u].x + B[u].x * p[u].y + B[u].y * p[u].z,
+                             B[u].z * p[u].x + B[u].w * p[u].y + C[u] * p[u].z);
+                R[0] += A[u].x; R[1] += A[u].y; R[2] += A[u].z; R[3] += A[u].w; R[4] += B[u].x;
+                R[5] += B[u].y; R[6] += B[u].z; R[7] += B[u].w; R[8] += C[u];
+            }
     }
     float3 r = ld3(rb, row);
     float3 rt = f3(R[0] * r.x + R[3] * r.y + R[6] * r.z, R[1] * r.x + R[4] * r.y + R[7] * r.z,
@@ -645,6 +687,12 @@ int ensure_adjoint_scratch(Handle& h) {
     return code;
 }
 
+// A kernel chained to the ones before it while its grid is small (kChainedBlocks).
+template <class... Params, class... Args>
+cudaError_t launch_small_chained(void (*kernel)(Params...), int blocks, int threads, cudaStream_t s, Args&&... args) {
+    return fem::launch_maybe_chained(blocks <= (int)fem::kChainedBlocks, kernel, blocks, threads, 0, s, args...);
+}
+
 // Element and node VJPs of the force terms at the packed state (h.q4, h.v4) for
 // the force gradient gs * g.  Per-element outputs are written, or accumulated
 // when `accumulate`; ext_bar (optional) accumulates gs * g; with zero_fixed the
@@ -654,15 +702,15 @@ cudaError_t launch_force_vjp(Handle& h, const float* activations, const float* g
                              float* hex_mat_bar, float* ext_bar, bool accumulate, bool zero_fixed, cudaStream_t s) {
     const int acc = accumulate ? 1 : 0;
     if (h.T > 0)
-        fem::tet_force_vjp_kernel<<<(h.T + 127) / 128, 128, 0, s>>>(
+        launch_small_chained(fem::tet_force_vjp_kernel, (h.T + 127) / 128, 128, s,
             h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.mu_scale, h.q4, h.v4, h.enable_act ? activations : nullptr, g,
             gs, h.min_stretch, h.max_stretch, h.elem_grad, act_bar, scale_bar, tet_mat_bar, acc);
     if (h.H > 0)
-        fem::hex_force_vjp_kernel<<<(int)((8 * (int64_t)h.H + 255) / 256), 256, 0, s>>>(
+        launch_small_chained(fem::hex_force_vjp_kernel, (int)((8 * (int64_t)h.H + 255) / 256), 256, s,
             h.H, h.hex_idx, h.hex_invJ, h.hex_detw, h.hex_mat, h.q4, h.v4, g, gs, h.min_stretch, h.max_stretch,
             h.elem_grad + 2 * 4 * (size_t)h.T, hex_mat_bar, acc);
     if (h.Tri > 0)
-        fem::tri_force_vjp_kernel<<<(h.Tri + 127) / 128, 128, 0, s>>>(
+        launch_small_chained(fem::tri_force_vjp_kernel, (h.Tri + 127) / 128, 128, s,
             h.Tri, h.tri_idx, h.tri_pose, h.tri_mat, h.q4, h.v4, g, gs,
             h.elem_grad + 2 * (4 * (size_t)h.T + 8 * (size_t)h.H));
     cudaError_t err = cudaGetLastError();
@@ -702,14 +750,16 @@ cudaError_t launch_force_vjp(Handle& h, const float* activations, const float* g
     a.ext_bar = ext_bar;
     a.q_bar = q_bar;
     a.v_bar = v_bar;
-    fem::node_vjp_kernel<<<(h.P + 127) / 128, 128, 0, s>>>(a);
+    launch_small_chained(fem::node_vjp_kernel, (h.P + 127) / 128, 128, s,
+            a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_predictor_vjp(Handle& h, const float* rhs_bar, float dt, float* v_bar, cudaStream_t s) {
     const int threads = 256;
     const int blocks = (h.nslices * 32 + threads - 1) / threads;
-    fem::predictor_vjp_kernel<<<blocks, threads, 0, s>>>(h.nslices, h.slice_ptr, h.slice_meta, h.row_info, h.valA,
+    launch_small_chained(fem::predictor_vjp_kernel, blocks, threads, s,
+            h.nslices, h.slice_ptr, h.slice_meta, h.row_info, h.valA,
                                                           h.valB, h.valC, h.scol, rhs_bar, h.node_spring_ptr,
                                                           h.node_spring_ent, h.spring_idx, h.spring_kd, dt, v_bar);
     return cudaGetLastError();
@@ -859,10 +909,12 @@ int fem_adjoint_segment(FemHandle* H, float* q_states, float* v_states, int32_t 
     cudaError_t err = refresh ? refresh_at(h, q_states, s) : cudaSuccess;
     float* rb = adjoint_start != nullptr ? adjoint_start : h.adj_x;  // the adjoint solution (and warm start)
     for (int k = substeps - 1; k >= 0 && err == cudaSuccess; --k) {
-        fem::adjoint_seed_kernel<<<blocks, threads, 0, s>>>(h.P, dt, h.fixed_mask, q_bar, v_bar, h.adj_vt);
+        launch_small_chained(fem::adjoint_seed_kernel, blocks, threads, s,
+            h.P, dt, h.fixed_mask, q_bar, v_bar, h.adj_vt);
         err = cudaGetLastError();
         if (err == cudaSuccess && adjoint_start != nullptr) {
-            fem::pack_adjoint_start_kernel<<<blocks, threads, 0, s>>>(h.P, rb, h.fixed_mask, h.x);
+            launch_small_chained(fem::pack_adjoint_start_kernel, blocks, threads, s,
+            h.P, rb, h.fixed_mask, h.x);
             err = cudaGetLastError();
         }
         if (err == cudaSuccess)

@@ -604,7 +604,6 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
     h.skf = d->soft_contact_kf;
     h.smu = d->soft_contact_mu;
     fem::upload_hex_reference_table();
-    fem::upload_hex_reference_table_adjoint();
 
     // ---- empty-material tets produce no triplets (kernels.py:690-700)
     std::vector<unsigned char> tet_empty(T, 0);

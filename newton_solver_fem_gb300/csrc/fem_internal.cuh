@@ -415,7 +415,6 @@ int report_cuda(cudaError_t err);
 // dN_a/dxi at the 8 Gauss points (host copy, filled as the reference computes it)
 void fill_hex_reference_table(float table[8][8][3]);
 void upload_hex_reference_table();          // fem_elements.cu copy
-void upload_hex_reference_table_adjoint();  // fem_adjoint.cu copy
 
 // --- launchers (fem_elements.cu) ---
 // zero_x: with pack_x, a zero warm start instead of dv

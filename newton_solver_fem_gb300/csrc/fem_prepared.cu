@@ -67,16 +67,33 @@ __global__ void predictor_diag_kernel(int nslices, const int* __restrict__ slice
     const float3 vi = xyz(v4[row]);
     float3 acc = f3(0.f, 0.f, 0.f);
     float d[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int k = 0; k < len; ++k) {
-        const size_t e = (size_t)(slice_ptr[sl] + k) * kSlice + lane;
-        const float4 a = valA[e], b = valB[e];
-        const float c = valC[e];
-        const int j = scol[e];
-        acc = acc + block_mul(a, b, c, xyz(v4[j]) - vi);
-        if (j == row) {
-            d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w;
-            d[4] = b.x; d[5] = b.y; d[6] = b.z; d[7] = b.w; d[8] = c;
+    // kColumnBatch blocks (and then their columns' velocities) in flight before any is used
+    constexpr int kColumnBatch = 4;
+    const int base = slice_ptr[sl];
+    for (int k0 = 0; k0 < len; k0 += kColumnBatch) {
+        float4 a[kColumnBatch], b[kColumnBatch];
+        float c[kColumnBatch];
+        int j[kColumnBatch];
+#pragma unroll
+        for (int u = 0; u < kColumnBatch; ++u) {
+            const size_t e = (size_t)(base + min(k0 + u, len - 1)) * kSlice + lane;
+            a[u] = valA[e];
+            b[u] = valB[e];
+            c[u] = valC[e];
+            j[u] = scol[e];
         }
+        float3 v[kColumnBatch];
+#pragma unroll
+        for (int u = 0; u < kColumnBatch; ++u) v[u] = xyz(v4[j[u]]);
+#pragma unroll
+        for (int u = 0; u < kColumnBatch; ++u)
+            if (k0 + u < len) {
+                acc = acc + block_mul(a[u], b[u], c[u], v[u] - vi);
+                if (j[u] == row) {
+                    d[0] = a[u].x; d[1] = a[u].y; d[2] = a[u].z; d[3] = a[u].w;
+                    d[4] = b[u].x; d[5] = b[u].y; d[6] = b[u].z; d[7] = b[u].w; d[8] = c[u];
+                }
+            }
     }
     if (info & kFixedBit) {
         for (int k = 0; k < 9; ++k) d[k] = (k % 4 == 0) ? 1.0f : 0.0f;
