@@ -1521,13 +1521,7 @@ int fem_export_bsr(FemHandle* H, int32_t* offsets, int32_t* columns, float* valu
     Handle& h = H->h;
     DeviceGuard g(H->device);
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t err = cudaSuccess;
-    if (offsets && h.P > 0)
-        err = cudaMemcpyAsync(offsets, h.bsr_offsets, sizeof(int) * (h.P + 1), cudaMemcpyDeviceToDevice, s);
-    if (err == cudaSuccess && columns && h.nnzb > 0)
-        err = cudaMemcpyAsync(columns, h.bsr_columns, sizeof(int) * h.nnzb, cudaMemcpyDeviceToDevice, s);
-    if (err == cudaSuccess && values) err = fem::launch_export_bsr(h, values, s);
-    return cuda_status(err, &h);
+    return cuda_status(fem::launch_export_bsr(h, offsets, columns, values, s), &h);
 }
 
 int fem_export_preconditioner(FemHandle* H, float* inverse_blocks, void* stream) {

@@ -121,11 +121,20 @@ constexpr int kExportRow = 9 * kExportColumns + 1;  // padded: the 32 rows of a 
 
 __global__ void __launch_bounds__(32 * kExportWarps) export_bsr_kernel(
     int nslices, const int* __restrict__ slice_ptr, const int2* __restrict__ meta, const unsigned* __restrict__ row_info,
-    const int* __restrict__ offsets, const float4* __restrict__ valA, const float4* __restrict__ valB,
-    const float* __restrict__ valC, float* __restrict__ out) {
+    const int* __restrict__ offsets, const int* __restrict__ columns, int64_t nnzb, int P,
+    const float4* __restrict__ valA, const float4* __restrict__ valB, const float* __restrict__ valC,
+    int* __restrict__ out_offsets, int* __restrict__ out_columns, float* __restrict__ out) {
     __shared__ float tile[kExportWarps][32 * kExportRow];
+    if (blockIdx.y == 0) {  // the pattern, in the same launch as the values (two device copies took 8 us)
+        const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+        if (out_offsets != nullptr)
+            for (int64_t i = i0; i <= P; i += step) out_offsets[i] = offsets[i];
+        if (out_columns != nullptr)
+            for (int64_t i = i0; i < nnzb; i += step) out_columns[i] = columns[i];
+        return;
+    }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int sl = blockIdx.x * kExportWarps + w, k0 = blockIdx.y * kExportColumns;
+    const int sl = blockIdx.x * kExportWarps + w, k0 = (blockIdx.y - 1) * kExportColumns;
     if (sl >= nslices) return;  // the whole warp
     const int base = slice_ptr[sl];
     if (base + k0 >= slice_ptr[sl + 1]) return;
@@ -164,11 +173,13 @@ cudaError_t launch_gather(Handle& h, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_export_bsr(Handle& h, float* values, cudaStream_t s) {
-    if (h.nnzb == 0) return cudaSuccess;
-    const dim3 grid(blocks_for(h.nslices, kExportWarps), blocks_for(h.slice_width, kExportColumns));
-    export_bsr_kernel<<<grid, 32 * kExportWarps, 0, s>>>(
-        h.nslices, h.slice_ptr, h.slice_meta, h.row_info, h.bsr_offsets, h.valA, h.valB, h.valC, values);
+cudaError_t launch_export_bsr(Handle& h, int* offsets, int* columns, float* values, cudaStream_t s) {
+    if (h.nslices == 0) return cudaSuccess;
+    const dim3 grid(blocks_for(h.nslices, kExportWarps),
+                    1 + (values != nullptr ? blocks_for(h.slice_width, kExportColumns) : 0));
+    export_bsr_kernel<<<grid, 32 * kExportWarps, 0, s>>>(h.nslices, h.slice_ptr, h.slice_meta, h.row_info,
+                                                         h.bsr_offsets, h.bsr_columns, h.nnzb, h.P, h.valA, h.valB,
+                                                         h.valC, offsets, columns, values);
     return cudaGetLastError();
 }
 

@@ -462,7 +462,8 @@ cudaError_t launch_soft_contacts(Handle& h, cudaStream_t s);      // per-contact
 cudaError_t launch_element_tangent(Handle& h, float dt, cudaStream_t s);
 // --- launchers (fem_assembly.cu) ---
 cudaError_t launch_gather(Handle& h, cudaStream_t s);
-cudaError_t launch_export_bsr(Handle& h, float* values, cudaStream_t s);
+// offsets, columns and values are each optional
+cudaError_t launch_export_bsr(Handle& h, int* offsets, int* columns, float* values, cudaStream_t s);
 cudaError_t launch_export_triplets(Handle& h, float* values, cudaStream_t s);
 // --- launchers (fem_pcg.cu) ---
 // Lets `kernel` launch with up to `bytes` of dynamic shared memory on the current device.  The limit is
