@@ -506,97 +506,59 @@ __device__ __forceinline__ void upper_pair(int u, int& a, int& b) {
 }
 
 constexpr int kTetTangentThreads = 128;
-constexpr int kTetFactor = 40;
+static_assert(kTetTangentThreads % kTetGroup == 0 && kTetGroup == 32, "a warp's tets are one group");
 
-// Reference kernels.py:635-850.  Phase 1: one thread per tet computes the
-// per-tet factors (F dm_a, dJ/dx_a, dm_a and three coefficients) into shared
-// memory.  Phase 2: 10 consecutive threads write the 10 blocks a <= b of a tet,
-// so the block run of each element is written contiguously.
+// Reference kernels.py:635-850.  One thread per tet: its factors (F dm_a, dJ/dx_a, dm_a and three
+// coefficients) stay in registers and it forms its ten blocks a <= b from them; a warp's stores of one
+// block are a run of 32.
 __global__ void __launch_bounds__(kTetTangentThreads) tet_tangent_kernel(
     int T, const int4* __restrict__ idx, const float* __restrict__ pose, const float* __restrict__ mat,
     const float* __restrict__ mu_scale, const float4* __restrict__ q4, float lo, float hi, float dt, int64_t trip_off,
     TripletPlanes vals) {
     chained_start();
-    __shared__ float sm[kTetTangentThreads][kTetFactor + 1];
-    int lt = threadIdx.x;
-    int t = blockIdx.x * kTetTangentThreads + lt;
-    float* fct = sm[lt];
-    if (t < T) {
-        float k_mu = mat[3 * t], k_lambda = mat[3 * t + 1];
-        if (mu_scale != nullptr) k_mu *= mu_scale[t];
-        if (k_mu == 0.0f && k_lambda == 0.0f && mat[3 * t + 2] == 0.0f) {
-            fct[39] = 2.0f;  // empty material: rows/cols are -1, nothing to write
-        } else {
-            M3 Dm;
+    const int t = blockIdx.x * kTetTangentThreads + threadIdx.x;
+    if (t >= T) return;
+    const int64_t ti = trip_off + (int64_t)(t / kTetGroup) * (10 * kTetGroup) + t % kTetGroup;
+    float k_mu = mat[3 * t], k_lambda = mat[3 * t + 1];
+    if (mu_scale != nullptr) k_mu *= mu_scale[t];
+    if (k_mu == 0.0f && k_lambda == 0.0f && mat[3 * t + 2] == 0.0f)
+        return;  // empty material: rows/cols are -1, nothing to write
+    M3 Dm;
 #pragma unroll
-            for (int k = 0; k < 9; ++k) Dm.m[k / 3][k % 3] = pose[9 * t + k];
-            float inv_rest_volume = det3(Dm) * 6.0f;
-            if (inv_rest_volume <= 0.0f) {
-                fct[39] = 1.0f;  // degenerate rest pose: zero blocks at valid rows
-            } else {
-                int4 n = idx[t];
-                float3 x0 = xyz(q4[n.x]), x1 = xyz(q4[n.y]), x2 = xyz(q4[n.z]), x3 = xyz(q4[n.w]);
-                float3 x10 = x1 - x0, x20 = x2 - x0, x30 = x3 - x0;
-                float rest_volume = 1.0f / inv_rest_volume;
-                float mu = k_mu * rest_volume, lam = k_lambda * rest_volume;
-                M3 F = clamp_stretch(matmul(from_cols(x10, x20, x30), Dm), lo, hi);
-                float3 c0 = col(F, 0), c1 = col(F, 1), c2 = col(F, 2);
-                float Ic = dot3(c0, c0) + dot3(c1, c1) + dot3(c2, c2);
-                float Ic1 = fmaxf(Ic + 1.0f, 1e-6f);
-                float s = 1.0f - 1.0f / Ic1;
-                float coef = mu * 2.0f / (Ic1 * Ic1);
-                float sv = inv_rest_volume / 6.0f;
-                float3 d1 = cross3(x20, x30) * sv, d2 = cross3(x30, x10) * sv, d3 = cross3(x10, x20) * sv;
-                float3 d0 = -(d1 + d2 + d3);
-                float3 m1 = row(Dm, 0), m2 = row(Dm, 1), m3 = row(Dm, 2);
-                float3 m0 = -(m1 + m2 + m3);
-                float3 dJ[4] = {d0, d1, d2, d3};
-                float3 dm[4] = {m0, m1, m2, m3};
-#pragma unroll
-                for (int a = 0; a < 4; ++a) {
-                    float3 fd = mul(F, dm[a]);
-                    fct[3 * a] = fd.x; fct[3 * a + 1] = fd.y; fct[3 * a + 2] = fd.z;
-                    fct[12 + 3 * a] = dJ[a].x; fct[13 + 3 * a] = dJ[a].y; fct[14 + 3 * a] = dJ[a].z;
-                    fct[24 + 3 * a] = dm[a].x; fct[25 + 3 * a] = dm[a].y; fct[26 + 3 * a] = dm[a].z;
-                }
-                fct[36] = mu * s;
-                fct[37] = coef;
-                fct[38] = lam;
-                fct[39] = 0.0f;
-            }
-        }
+    for (int k = 0; k < 9; ++k) Dm.m[k / 3][k % 3] = pose[9 * t + k];
+    float inv_rest_volume = det3(Dm) * 6.0f;
+    if (inv_rest_volume <= 0.0f) {  // degenerate rest pose: zero blocks at valid rows
+        const float o[9] = {};
+        for (int u = 0; u < 10; ++u) store_block(vals, ti + u * kTetGroup, o);
+        return;
     }
-    __syncthreads();
-    float scale = dt * dt;
-#pragma unroll 2
-    for (int m = 0; m < 10; ++m) {
-        int b = lt + kTetTangentThreads * m;
-        int le = b / 10, ab = b - 10 * le;
-        int te = blockIdx.x * kTetTangentThreads + le;
-        if (te >= T) continue;
-        const float* f = sm[le];
-        float mode = f[39];
-        if (mode == 2.0f) continue;
-        const int64_t ti = trip_off + 10 * (int64_t)te + ab;
-        float o[9];
-        if (mode == 1.0f) {
+    int4 n = idx[t];
+    float3 x0 = xyz(q4[n.x]), x1 = xyz(q4[n.y]), x2 = xyz(q4[n.z]), x3 = xyz(q4[n.w]);
+    float3 x10 = x1 - x0, x20 = x2 - x0, x30 = x3 - x0;
+    float rest_volume = 1.0f / inv_rest_volume;
+    float mu = k_mu * rest_volume, lam = k_lambda * rest_volume;
+    M3 F = clamp_stretch(matmul(from_cols(x10, x20, x30), Dm), lo, hi);
+    float3 c0 = col(F, 0), c1 = col(F, 1), c2 = col(F, 2);
+    float Ic = dot3(c0, c0) + dot3(c1, c1) + dot3(c2, c2);
+    float Ic1 = fmaxf(Ic + 1.0f, 1e-6f);
+    float s = 1.0f - 1.0f / Ic1;
+    const float coef = mu * 2.0f / (Ic1 * Ic1), mus = mu * s, scale = dt * dt;
+    float sv = inv_rest_volume / 6.0f;
+    float3 d1 = cross3(x20, x30) * sv, d2 = cross3(x30, x10) * sv, d3 = cross3(x10, x20) * sv;
+    float3 m1 = row(Dm, 0), m2 = row(Dm, 1), m3 = row(Dm, 2);
+    const float3 dJ[4] = {-(d1 + d2 + d3), d1, d2, d3};
+    const float3 dm[4] = {-(m1 + m2 + m3), m1, m2, m3};
+    float3 fd[4];
 #pragma unroll
-            for (int k = 0; k < 9; ++k) o[k] = 0.0f;
-            store_block(vals, ti, o);
-            continue;
-        }
-        int a, bb;
-        upper_pair(ab, a, bb);
-        float3 Fa = f3(f[3 * a], f[3 * a + 1], f[3 * a + 2]);
-        float3 Fb = f3(f[3 * bb], f[3 * bb + 1], f[3 * bb + 2]);
-        float3 Ja = f3(f[12 + 3 * a], f[13 + 3 * a], f[14 + 3 * a]);
-        float3 Jb = f3(f[12 + 3 * bb], f[13 + 3 * bb], f[14 + 3 * bb]);
-        float3 ma = f3(f[24 + 3 * a], f[25 + 3 * a], f[26 + 3 * a]);
-        float3 mb = f3(f[24 + 3 * bb], f[25 + 3 * bb], f[26 + 3 * bb]);
-        float diag = f[36] * dot3(ma, mb);
-        float coef = f[37], lam = f[38];
-        float fa[3] = {Fa.x, Fa.y, Fa.z}, fb[3] = {Fb.x, Fb.y, Fb.z};
-        float ja[3] = {Ja.x, Ja.y, Ja.z}, jb[3] = {Jb.x, Jb.y, Jb.z};
+    for (int a = 0; a < 4; ++a) fd[a] = mul(F, dm[a]);
+#pragma unroll
+    for (int u = 0; u < 10; ++u) {
+        int a, b;
+        upper_pair(u, a, b);
+        const float diag = mus * dot3(dm[a], dm[b]);
+        const float fa[3] = {fd[a].x, fd[a].y, fd[a].z}, fb[3] = {fd[b].x, fd[b].y, fd[b].z};
+        const float ja[3] = {dJ[a].x, dJ[a].y, dJ[a].z}, jb[3] = {dJ[b].x, dJ[b].y, dJ[b].z};
+        float o[9];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -605,7 +567,7 @@ __global__ void __launch_bounds__(kTetTangentThreads) tet_tangent_kernel(
                 float kvol = ja[i] * jb[j] * lam;
                 o[3 * i + j] = (kdev + kvol) * scale;
             }
-        store_block(vals, ti, o);
+        store_block(vals, ti + u * kTetGroup, o);
     }
 }
 
@@ -1007,12 +969,11 @@ cudaError_t launch_constant_blocks(Handle& h, float dt, cudaStream_t s) {
 }
 
 cudaError_t launch_element_tangent(Handle& h, float dt, cudaStream_t s) {
-    int64_t tet_off = tet_triplet_offset(h);
     if (h.T > 0)
         launch_maybe_chained(
             blocks_for(h.T, kTetTangentThreads) <= (int)kChainedBlocks, tet_tangent_kernel,
-            blocks_for(h.T, kTetTangentThreads), kTetTangentThreads, 0, s, h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.mu_scale, h.q4, h.min_stretch, h.max_stretch, dt, tet_off,
-            h.trip);
+            blocks_for(h.T, kTetTangentThreads), kTetTangentThreads, 0, s, h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.mu_scale, h.q4, h.min_stretch, h.max_stretch, dt,
+            h.trip_map.tet_start(), h.trip);
     if (h.H > 0) {
         cudaError_t err = allow_dynamic_smem((const void*)hex_tangent_kernel, kTanSmemBytes);
         if (err != cudaSuccess) return err;

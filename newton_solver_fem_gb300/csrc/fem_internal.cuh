@@ -33,14 +33,19 @@ struct TripletPlanes {
 // Where the planes hold a triplet.  Element matrices are exactly symmetric (the kernels form K_ba as the
 // transpose of K_ab, term by term), so only the blocks a <= b are stored: 10 of a tet's 16 and 36 of a
 // hex's 64; a block below the diagonal is read transposed.  That is 0.56 of the bytes the tangent
-// kernels write and the assembly reads.  The hexes are stored in groups of 16 (one tangent CTA), block
-// by block over the group's hexes: a CTA's output is one run per plane, and a slice's rows, which touch
-// consecutive hexes at a block, read consecutive entries.
+// kernels write and the assembly reads.  The elements are stored in groups, block by block over the
+// group's elements: hexes by 16 (one tangent CTA: its output is one run per plane), tets by 32 (a warp,
+// a thread each), so that a store is a run, and a slice's rows, which touch neighbouring elements at a
+// block, read neighbouring entries.
 constexpr int kHexGroup = 16;
+constexpr int kTetGroup = 32;
 struct TripletMap {
     int64_t constants = 0;  // [P | 2S | 3Tri], stored as they are
     int64_t tets = 0, hexes = 0;
-    __host__ __device__ __forceinline__ int64_t hex_start() const { return (constants + 10 * tets + 3) & ~(int64_t)3; }
+    __host__ __device__ __forceinline__ int64_t tet_start() const { return (constants + 7) & ~(int64_t)7; }
+    __host__ __device__ __forceinline__ int64_t hex_start() const {
+        return tet_start() + 10 * kTetGroup * ((tets + kTetGroup - 1) / kTetGroup);
+    }
     __host__ __device__ __forceinline__ int64_t stored() const {
         return hex_start() + 36 * kHexGroup * ((hexes + kHexGroup - 1) / kHexGroup);
     }
@@ -56,7 +61,7 @@ struct TripletMap {
             const int u = lo * n - lo * (lo - 1) / 2 + (hi - lo);
             flip = a > b;
             at = hex ? hex_start() + (e / kHexGroup) * (36 * kHexGroup) + u * kHexGroup + e % kHexGroup
-                     : constants + 10 * e + u;
+                     : tet_start() + (e / kTetGroup) * (10 * kTetGroup) + u * kTetGroup + e % kTetGroup;
         }
         return (unsigned)(at << 1) | flip;
     }
