@@ -172,7 +172,8 @@ int fem_set_wait_limit(FemHandle* handle, int64_t nanoseconds);
 
 /* Launch tuning of the persistent PCG kernel (chosen by an autotuner).  Not
  * capturable: a change rebuilds the launch tables. */
-#define FEM_TUNE_SPMV_UNROLL 1       /* block columns in flight per thread: 1, 2 or 4 (default 4) */
+#define FEM_TUNE_SPMV_UNROLL 1       /* block columns in flight per thread: 1, 2 or 4 (default: 4 while the matrix
+                                      * stays in L2 between CG iterations, else 2); read: what is in use */
 #define FEM_TUNE_L2_RESIDENT_BYTES 2 /* matrix bytes loaded evict_last (kept in L2 across iterations); -1 = 60% of L2;
                                         -2 (default) = the whole matrix when it fits in 60% of L2, else none */
 #define FEM_TUNE_RESIDENT_SLICES 3   /* read-only: resulting number of L2-resident 32-row slices */

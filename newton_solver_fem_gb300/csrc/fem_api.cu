@@ -1394,7 +1394,7 @@ int fem_get_tuning(FemHandle* H, int32_t key, int64_t* value) {
     if (H == nullptr || value == nullptr) return set_error(FEM_ERR_BAD_ARG, "null handle or output");
     Handle& h = H->h;
     switch (key) {
-        case FEM_TUNE_SPMV_UNROLL: *value = h.spmv_unroll; return FEM_OK;
+        case FEM_TUNE_SPMV_UNROLL: *value = h.spmv_unroll_used; return FEM_OK;
         case FEM_TUNE_L2_RESIDENT_BYTES: *value = h.l2_resident_bytes; return FEM_OK;
         case FEM_TUNE_RESIDENT_SLICES: *value = h.resident_slices; return FEM_OK;
         case FEM_TUNE_GRID: *value = h.grid; return FEM_OK;

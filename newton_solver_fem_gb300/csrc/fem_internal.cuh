@@ -208,7 +208,8 @@ struct Handle {
     int enable_act = 0, precond = 0, maxiter = 50;
     float tol = 1e-2f;
     long long wait_limit_ns = 2000000000LL;
-    int spmv_unroll = 4;          // block columns in flight per thread in the PCG SpMV (1, 2 or 4)
+    int spmv_unroll = 0;          // requested block columns in flight per thread in the PCG SpMV: 1, 2, 4 or 0 (automatic)
+    int spmv_unroll_used = 4;     // and what the launch configuration chose
     int64_t l2_resident_bytes = -2;  // matrix bytes loaded evict_last (-1: 60% of L2; -2: all if it fits there, else 0)
     int pcg_threads = 0;             // threads per PCG CTA (256, 512, 1024; 0 = chosen from the problem size)
     int balance = 0;                 // 1: slices split by calibrated per-CTA speed (FEM_TUNE_BALANCE)
@@ -502,7 +503,7 @@ cudaError_t launch_pcg_onchip(Handle& h, float dt, int write_state, float* q_out
 inline bool onchip_in_use(const Handle& h) {
     if (h.oc_grid == 0 || h.onchip == 0 || h.cg_variant != 0 || h.balance != 0) return false;
     return h.onchip == 1 || (h.pcg_threads == 0 && h.grid_cap == 0 && h.resident_pref == -1 && h.compact_cols == -1 &&
-                             h.l2_resident_bytes == -2 && h.spmv_unroll == 4 && h.tail_prefetch == 50 &&
+                             h.l2_resident_bytes == -2 && h.spmv_unroll == 0 && h.tail_prefetch == 50 &&
                              h.split_headroom == 0);
 }
 // Step mode (solve_rhs == nullptr): predictor, normalised PCG from the dv warm start, integration.

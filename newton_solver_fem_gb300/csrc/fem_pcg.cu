@@ -155,12 +155,23 @@ __device__ __forceinline__ Entry load_entry(const PcgArgs& a, size_t e, int k, i
     return m;
 }
 
+// A node's (z, p) record in one 32-byte load: half the load instructions and L1 accesses of two float4
+// loads.  The record buffers start on an allocation boundary, so every record is 32-byte aligned.
+__device__ __forceinline__ void ld_record(const float4* rec, float4& z, float4& p) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(z.x), "=f"(z.y), "=f"(z.z), "=f"(z.w), "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w)
+                 : "l"(rec)
+                 : "memory");
+}
+
 // p_j = z_j (first iteration) or z_j + beta p_j from record buffer rec.
 template <bool FIRST>
 __device__ __forceinline__ float3 gather_p(const float4* rec, int j, float beta) {
     const float4* q = rec + 2 * (size_t)j;
     if (FIRST) return xyz(q[0]);
-    return next_p(q[0], q[1], beta);
+    float4 z, p;
+    ld_record(q, z, p);
+    return next_p(z, p, beta);
 }
 
 // y_row = sum_k A_k p_{j_k}, with p = z (first iteration) or z + beta p_old.
@@ -1025,7 +1036,12 @@ cudaError_t pcg_configure(Handle& h) {
     if (!coop) return cudaErrorNotSupported;
     const int cm = column_mode(h);
     const int V = h.cg_variant;
-    PcgKernel kern = pcg_kernel_for(h.spmv_unroll, cm, V);
+    // Automatic blocks in flight per thread: 4 while the matrix stays in L2 between iterations (latency is
+    // what counts: 17.3 against 19.3 us per iteration on 68,921 Hex8 nodes), 2 when it streams from DRAM,
+    // where more requests from each of 4,864 warps only break up the runs that DRAM serves (64^3 Hex8: 54.2
+    // against 57.7 us; 72^3 Tet4 48.6 against 52.5).
+    h.spmv_unroll_used = h.spmv_unroll > 0 ? h.spmv_unroll : (h.resident_slices < h.nslices ? 2 : 4);
+    PcgKernel kern = pcg_kernel_for(h.spmv_unroll_used, cm, V);
     // Automatic CTA size: 1024-thread CTAs once there are 8 slices per SM (fewer
     // CTAs make the grid reductions cheaper: on a 3,677-slice Tet4 system 115
     // such CTAs beat 460 of 256 threads by 8% per CG iteration); small systems
@@ -1045,6 +1061,11 @@ cudaError_t pcg_configure(Handle& h) {
         int grid, L, stage, resident;
         size_t smem;
     };
+    // Shared memory that row state may take when it was not asked for: the rest of the SM's 256 KB is the L1
+    // that the column gathers hit.  Hex8 batch of 48 scenes (79 slices per CTA): 58.0 us per iteration with
+    // 193 KB of state, 46.6 with 102 KB; 90^3 Hex8 (155 slices): 185 with 200 KB of staging, 144 without;
+    // up to 140 KB the state is the faster one (56^3: 42.1 against 43.5 and 44.7).
+    const size_t state_limit = (h.resident_pref < 0 ? 160 : 227) * 1024;
     auto fit = [&](int want_resident, int slack_pct, Config& c) -> cudaError_t {
         int grid = (h.nslices + warps_per_cta - 1) / warps_per_cta;
         // wide CTAs on a system too small to give every SM one slice per warp:
@@ -1067,7 +1088,7 @@ cudaError_t pcg_configure(Handle& h) {
                 if ((lay.st | lay.tot | lay.segb | lay.sseg | lay.slc | lay.kmask | lay.kval | lay.rinfo | lay.stage |
                      lay.res) & 15)
                     return cudaErrorMisalignedAddress;
-                if (lay.total > 227 * 1024) {
+                if (lay.total > (res || stage ? state_limit : (size_t)227 * 1024)) {
                     per_sm = 0;
                 } else {
                     cudaError_t e = allow_dynamic_smem((const void*)kern, lay.total);
@@ -1201,7 +1222,7 @@ cudaError_t launch_pcg(Handle& h, float dt, int write_state, float* q_out, float
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, pcg_kernel_for(h.spmv_unroll, cm, h.cg_variant), a);
+    return cudaLaunchKernelEx(&cfg, pcg_kernel_for(h.spmv_unroll_used, cm, h.cg_variant), a);
 }
 
 }  // namespace fem
