@@ -8,6 +8,8 @@
 // in order: no atomics, bit-identical results run to run.  The thread that
 // owns a diagonal slot also writes that row's preconditioner block
 // (kernels.py:1836-1849 fused into the assembly epilogue).
+#include <algorithm>
+
 #include "fem_internal.cuh"
 #include "fem_math.cuh"
 
@@ -111,30 +113,89 @@ __global__ void export_triplets_kernel(int64_t ntrip, const TripletMap map, cons
     o[8] = trip.c[t];
 }
 
-// The SELL blocks as BSR values (rows ascending, a row's columns in its SELL order), 36 bytes a block.
-// A warp takes kExportColumns block columns of a slice (blockIdx.y): the planes are read coalesced into
-// shared memory, and each row's run of blocks, contiguous in BSR order, is written by the whole warp (a
-// thread per block wrote 4 bytes every 36: 115 us for 3.05 million blocks, 64 with a warp walking a
-// whole slice).
+// The matrix in BSR form: the pattern, and the SELL blocks as values (rows ascending, a row's columns in
+// its SELL order), 36 bytes a block.  The rows of a slice are one run of BSR values, so a CTA reads the
+// slice's planes coalesced, places the blocks in that order in shared memory and writes the run with one
+// bulk copy (its ends, up to a 16-byte boundary, by single stores).  3.05 million blocks take 52 us; 62
+// with a warp storing each row's run of eight columns, 115 with a thread per block.  The first
+// pattern_blocks CTAs copy the pattern (two device copies after the kernel took 8 us).
+constexpr int kExportThreads = 128, kExportMaxWidth = 64;
+
+struct ExportArgs {
+    int pattern_blocks;
+    const int* __restrict__ slice_ptr;
+    const int2* __restrict__ meta;
+    const unsigned* __restrict__ row_info;
+    const int* __restrict__ offsets;
+    const int* __restrict__ columns;
+    int64_t nnzb;
+    int P;
+    const float4* __restrict__ valA;
+    const float4* __restrict__ valB;
+    const float* __restrict__ valC;
+    int* __restrict__ out_offsets;
+    int* __restrict__ out_columns;
+    float* __restrict__ out;
+};
+
+__global__ void __launch_bounds__(kExportThreads) export_bsr_kernel(const ExportArgs a) {
+    extern __shared__ __align__(16) float tile[];
+    if ((int)blockIdx.x < a.pattern_blocks) {
+        const int64_t i0 = (int64_t)blockIdx.x * kExportThreads + threadIdx.x;
+        const int64_t step = (int64_t)a.pattern_blocks * kExportThreads;
+        if (a.out_offsets != nullptr)
+            for (int64_t i = i0; i <= a.P; i += step) a.out_offsets[i] = a.offsets[i];
+        if (a.out_columns != nullptr)
+            for (int64_t i = i0; i < a.nnzb; i += step) a.out_columns[i] = a.columns[i];
+        return;
+    }
+    const int sl = blockIdx.x - a.pattern_blocks;
+    const int lane = threadIdx.x & 31;
+    const int base = a.slice_ptr[sl], width = a.slice_ptr[sl + 1] - base;
+    const int2 m = a.meta[sl];
+    const int run0 = a.offsets[m.x], run1 = a.offsets[m.x + m.y];
+    const bool live = lane < m.y;
+    const int len = live ? (int)(a.row_info[m.x + lane] & ~kFixedBit) : 0;
+    float* out = a.out + 9 * (size_t)run0;
+    const int shift = (int)((reinterpret_cast<uintptr_t>(out) >> 2) & 3);  // of both copies, in floats
+    float* t = tile + shift;
+    float* row = t + 9 * (live ? a.offsets[m.x + lane] - run0 : 0);
+#pragma unroll 4
+    for (int k = threadIdx.x >> 5; k < width; k += kExportThreads / 32)
+        if (k < len) {
+            const size_t e = (size_t)(base + k) * kSlice + lane;
+            const float4 va = __ldg(a.valA + e), vb = __ldg(a.valB + e);
+            float* o = row + 9 * k;
+            o[0] = va.x; o[1] = va.y; o[2] = va.z; o[3] = va.w;
+            o[4] = vb.x; o[5] = vb.y; o[6] = vb.z; o[7] = vb.w;
+            o[8] = __ldg(a.valC + e);
+        }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the placed blocks visible to the bulk copy
+    __syncthreads();
+    const int n = 9 * (run1 - run0), head = min(n, (4 - shift) & 3), bulk = (n - head) & ~3;
+    if (threadIdx.x == 0 && bulk > 0) {
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out + head),
+                     "r"((unsigned)__cvta_generic_to_shared(t + head)), "r"(4 * bulk)
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+    if ((int)threadIdx.x - 32 >= 0 && (int)threadIdx.x - 32 < head) out[threadIdx.x - 32] = t[threadIdx.x - 32];
+    const int tail = head + bulk + (int)threadIdx.x - 64;
+    if (threadIdx.x >= 64 && tail < n) out[tail] = t[tail];
+}
+
+// The same for slices too wide for that: a warp takes kExportColumns block columns of a slice
+// (blockIdx.y) and writes each row's run of them (62 us for the 3.05 million blocks).
 constexpr int kExportColumns = 8, kExportWarps = 4;
 constexpr int kExportRow = 9 * kExportColumns + 1;  // padded: the 32 rows of a column in distinct banks
 
-__global__ void __launch_bounds__(32 * kExportWarps) export_bsr_kernel(
+__global__ void __launch_bounds__(32 * kExportWarps) export_columns_kernel(
     int nslices, const int* __restrict__ slice_ptr, const int2* __restrict__ meta, const unsigned* __restrict__ row_info,
-    const int* __restrict__ offsets, const int* __restrict__ columns, int64_t nnzb, int P,
-    const float4* __restrict__ valA, const float4* __restrict__ valB, const float* __restrict__ valC,
-    int* __restrict__ out_offsets, int* __restrict__ out_columns, float* __restrict__ out) {
+    const int* __restrict__ offsets, const float4* __restrict__ valA, const float4* __restrict__ valB,
+    const float* __restrict__ valC, float* __restrict__ out) {
     __shared__ float tile[kExportWarps][32 * kExportRow];
-    if (blockIdx.y == 0) {  // the pattern, in the same launch as the values (two device copies took 8 us)
-        const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
-        if (out_offsets != nullptr)
-            for (int64_t i = i0; i <= P; i += step) out_offsets[i] = offsets[i];
-        if (out_columns != nullptr)
-            for (int64_t i = i0; i < nnzb; i += step) out_columns[i] = columns[i];
-        return;
-    }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int sl = blockIdx.x * kExportWarps + w, k0 = (blockIdx.y - 1) * kExportColumns;
+    const int sl = blockIdx.x * kExportWarps + w, k0 = blockIdx.y * kExportColumns;
     if (sl >= nslices) return;  // the whole warp
     const int base = slice_ptr[sl];
     if (base + k0 >= slice_ptr[sl + 1]) return;
@@ -175,11 +236,35 @@ cudaError_t launch_gather(Handle& h, cudaStream_t s) {
 
 cudaError_t launch_export_bsr(Handle& h, int* offsets, int* columns, float* values, cudaStream_t s) {
     if (h.nslices == 0) return cudaSuccess;
-    const dim3 grid(blocks_for(h.nslices, kExportWarps),
-                    1 + (values != nullptr ? blocks_for(h.slice_width, kExportColumns) : 0));
-    export_bsr_kernel<<<grid, 32 * kExportWarps, 0, s>>>(h.nslices, h.slice_ptr, h.slice_meta, h.row_info,
-                                                         h.bsr_offsets, h.bsr_columns, h.nnzb, h.P, h.valA, h.valB,
-                                                         h.valC, offsets, columns, values);
+    const bool narrow = h.slice_width <= kExportMaxWidth;
+    ExportArgs a;
+    a.pattern_blocks = offsets != nullptr || columns != nullptr
+                           ? std::min(1024, blocks_for(std::max<int64_t>(h.nnzb, h.P + 1), 8 * kExportThreads))
+                           : 0;
+    a.slice_ptr = h.slice_ptr;
+    a.meta = h.slice_meta;
+    a.row_info = h.row_info;
+    a.offsets = h.bsr_offsets;
+    a.columns = h.bsr_columns;
+    a.nnzb = h.nnzb;
+    a.P = h.P;
+    a.valA = h.valA;
+    a.valB = h.valB;
+    a.valC = h.valC;
+    a.out_offsets = offsets;
+    a.out_columns = columns;
+    a.out = values;
+    const int slices = values != nullptr && narrow ? h.nslices : 0;
+    const size_t bytes = slices > 0 ? (9 * (size_t)h.slice_width * kSlice + 4) * sizeof(float) : 0;
+    if (a.pattern_blocks + slices > 0) {
+        cudaError_t err = allow_dynamic_smem((const void*)export_bsr_kernel, bytes);
+        if (err != cudaSuccess) return err;
+        export_bsr_kernel<<<a.pattern_blocks + slices, kExportThreads, bytes, s>>>(a);
+    }
+    if (values != nullptr && !narrow)
+        export_columns_kernel<<<dim3(blocks_for(h.nslices, kExportWarps), blocks_for(h.slice_width, kExportColumns)),
+                                32 * kExportWarps, 0, s>>>(h.nslices, h.slice_ptr, h.slice_meta, h.row_info,
+                                                           h.bsr_offsets, h.valA, h.valB, h.valC, values);
     return cudaGetLastError();
 }
 

@@ -586,3 +586,31 @@ def test_full_size_jittered_tet_block_with_springs_and_ground():
     q = to_np(a.particle_q)
     assert np.isfinite(q).all()
     assert q[:, 2].min() > -0.01  # the ground holds the block (penetration below 1 cm)
+
+
+@pytest.mark.parametrize("star", [0, 5, 56, 57])  # widest row: 18, 18, 64 and 65 block columns (64 is the run export's limit)
+def test_matrix_export_writes_the_assembled_blocks_and_nothing_else(star):
+    """The BSR export against the oracle's blocks, whole and in parts, at every 4-byte alignment of the values."""
+    x, hexes, mats, mass = scenes.hex_block(5, 3, 2, 0.1, (0.0, 0.0, 0.0), 2e4, 0.3, 1000.0)
+    n = len(x)
+    x = np.concatenate([x, 5.0 + np.arange(3 * star, dtype=float).reshape(star, 3)])
+    mass = np.concatenate([mass, np.full(star, 0.01)])
+    springs = np.stack([np.zeros(star, np.int64), n + np.arange(star)], 1) if star else None
+    kw = dict(springs=springs, spring_ke=np.full(star, 500.0), spring_kd=np.full(star, 1.0)) if star else {}
+    model, solver, oracle = make_pair(x, mass, hexes=hexes, hex_materials=mats, **kw)
+    q = rounded(deformed(oracle.rest))
+    solver.refresh_tangent(tensor(q))
+    oracle.refresh_tangent(q)
+    whole = solver.A_bsr
+    np.testing.assert_array_equal(whole.columns.cpu().numpy(), oracle.columns)
+    np.testing.assert_allclose(to_np(whole.values), oracle.values, rtol=0, atol=1e-5 * np.abs(oracle.values).max())
+    nv = whole.values.numel()
+    for off in range(4):
+        buf = torch.full((nv + 8,), 7.5, device=DEVICE)
+        part = buf[off:]
+        _lib.check(solver._lib.fem_export_bsr(solver._handle, None, None, part.data_ptr(), solver._stream()))
+        assert torch.equal(buf[off:off + nv], whole.values.flatten())
+        assert bool((buf[:off] == 7.5).all()) and bool((buf[off + nv:] == 7.5).all())
+    offsets = torch.full_like(whole.offsets, -1)
+    _lib.check(solver._lib.fem_export_bsr(solver._handle, offsets.data_ptr(), None, None, solver._stream()))
+    assert torch.equal(offsets, whole.offsets)
