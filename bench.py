@@ -820,7 +820,7 @@ def run_gb300(args) -> None:
                        "launch": launch_shape(solver),
                        "pcg_split": "rows split over CTAs by calibrated SpMV speed (FEM_TUNE_BALANCE=1)",
                        "column_mode": int(cc.value), "column_index_bytes": round(col_bytes, 4),
-                       "l2": "inputs larger than L2 (A values 259 MB, element blocks 614 MB at 64^3)"},
+                       "l2": "inputs larger than L2 (A values 259 MB, element blocks 350 MB at 64^3)"},
             "roofline": {"kernel": "pcg_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": peak_kind, "traffic": traffic,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of two full 64^3 launches "
