@@ -118,6 +118,29 @@ def test_automatic_residency_and_column_mode():
         assert lib.fem_set_tuning(solver._handle, key, bad) == _lib.FEM_ERR_BAD_ARG
 
 
+@pytest.mark.parametrize("cap,state", [(9, 1), (6, 0), (3, 0)])  # 55, 82 and 163 slices per CTA
+@pytest.mark.parametrize("l2_bytes,depth", [(-2, 4), (0, 2)])
+def test_automatic_depth_and_row_state_change_no_bit(cap, state, l2_bytes, depth):
+    """A matrix that streams is read two blocks at a time, one that stays in L2 four; row state is kept in
+    shared memory up to 160 KB unless it is asked for.  Neither changes the order of a sum."""
+    sc = scenes.hex_block_64(n=24)
+    model, solver, _ = scene_pair(sc, linear_solver_tolerance=1e-6, linear_solver_maxiter=100, with_oracle=False)
+    lib = _lib.load()
+    for key, value in ((_lib.FEM_TUNE_CTA_THREADS, 1024), (_lib.FEM_TUNE_GRID_CAP, cap),
+                       (_lib.FEM_TUNE_L2_RESIDENT_BYTES, l2_bytes)):
+        _lib.check(lib.fem_set_tuning(solver._handle, key, value))
+    assert setting(solver, _lib.FEM_TUNE_SPMV_UNROLL) == depth
+    assert setting(solver, _lib.FEM_TUNE_RESIDENT_STATE) == state
+    got = substep(model, solver, sc)
+    for key, value in ((_lib.FEM_TUNE_SPMV_UNROLL, 6 - depth), (_lib.FEM_TUNE_RESIDENT_LAYOUT, 1)):
+        _lib.check(lib.fem_set_tuning(solver._handle, key, value))
+    assert setting(solver, _lib.FEM_TUNE_SPMV_UNROLL) == 6 - depth
+    assert setting(solver, _lib.FEM_TUNE_RESIDENT_STATE) == (1 if cap > 3 else 0)
+    asked = substep(model, solver, sc)
+    for a, b in zip(got, asked):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_column_modes_are_bit_identical_and_report_shared_slots():
     """Column modes only change where a block's column comes from, so substeps agree bit for bit."""
     sc = scenes.hex_block_64(n=12)
