@@ -1037,9 +1037,10 @@ cudaError_t pcg_configure(Handle& h) {
     const int cm = column_mode(h);
     const int V = h.cg_variant;
     // Automatic blocks in flight per thread: 4 while the matrix stays in L2 between iterations (latency is
-    // what counts: 17.3 against 19.3 us per iteration on 68,921 Hex8 nodes), 2 when it streams from DRAM,
-    // where more requests from each of 4,864 warps only break up the runs that DRAM serves (64^3 Hex8: 54.2
-    // against 57.7 us; 72^3 Tet4 48.6 against 52.5).
+    // what counts: 17.3 against 19.3 us per iteration on 68,921 Hex8 nodes), 2 when it streams from DRAM
+    // (64^3 Hex8: 54.2 against 57.7 us; 72^3 Tet4 48.6 against 52.5; also with the next columns or whole
+    // column ranges requested ahead, more outstanding reads of a streamed matrix were slower, at the same
+    // DRAM bytes).
     h.spmv_unroll_used = h.spmv_unroll > 0 ? h.spmv_unroll : (h.resident_slices < h.nslices ? 2 : 4);
     PcgKernel kern = pcg_kernel_for(h.spmv_unroll_used, cm, V);
     // Automatic CTA size: 1024-thread CTAs once there are 8 slices per SM (fewer
