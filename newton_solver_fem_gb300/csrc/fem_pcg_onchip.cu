@@ -220,7 +220,10 @@ __device__ __forceinline__ void store_remote(const float* p, unsigned rank, floa
     asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\t"
                  "st.shared::cluster.f32 [r], %2;\n\t}" ::"r"(local), "r"(rank), "f"(v) : "memory");
 }
+// The aligned forms are executed by whole warps together, and callers come from loops whose trip counts differ
+// between lanes (a cluster's size and a halo's length are any number): the warp meets first.
 __device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 

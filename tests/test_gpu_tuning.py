@@ -274,6 +274,36 @@ def test_onchip_kernel_solves_the_streaming_kernels_system(element, cells):
         assert rel_l2(a, c) < 1e-5
 
 
+@pytest.mark.parametrize("layers,ctas", [(8, 5), (9, 6), (11, 7), (14, 9), (16, 10), (17, 11), (20, 13), (22, 14), (24, 15)])
+def test_onchip_clusters_of_any_size_solve_the_streaming_kernels_system(layers, ctas):
+    """Clusters whose size is no multiple of four, where the lanes that hand totals to the peers make unequal
+    numbers of trips before the cluster barrier: the launch variants' bound, and the same bits each time."""
+    from gpu_helpers import make_pair
+
+    x, hexes, mats, mass = scenes.hex_block(layers - 1, 4, 3, 0.01, (0.0, 0.0, 0.0), 2e5, 0.4, 1000.0)
+    order = np.random.default_rng(0).permutation(len(x))  # every slice holds a row of 27 blocks: past the one-CTA limit
+    x[order], mass[order], hexes = x.copy(), mass.copy(), order[hexes].astype(np.int32)
+    fixed = np.nonzero(np.isclose(x[:, 0], 0.0))[0].astype(np.int32)
+    model, solver, _ = make_pair(x, mass, fixed=fixed, hexes=hexes, hex_materials=mats, with_oracle=False,
+                                 linear_solver_tolerance=1e-6, linear_solver_maxiter=200)
+    lib = _lib.load()
+    rhs = torch.tensor((np.random.default_rng(37).normal(0.0, 1.0, x.shape) * mass[:, None]).astype(np.float32),
+                       device="cuda")
+
+    def run():
+        y = torch.empty_like(rhs)
+        _lib.check(lib.fem_solve(solver._handle, rhs.data_ptr(), y.data_ptr(), 1e-6, 200, solver._stream()))
+        torch.cuda.synchronize()
+        assert solver.stats()["status"] == 0
+        return to_np(y)
+
+    assert setting(solver, _lib.FEM_TUNE_ONCHIP_GRID) == ctas
+    got, again = run(), run()
+    _lib.check(lib.fem_set_tuning(solver._handle, _lib.FEM_TUNE_ONCHIP, 0))
+    np.testing.assert_array_equal(got, again)
+    assert rel_l2(got, run()) < 1e-5
+
+
 @pytest.mark.parametrize("count,dims", [(2, (2, 3)), (24, (3, 10)), (9, (2, 24)), (152, (2, 5))],
                          ids=lambda v: str(v).replace(" ", ""))
 def test_onchip_teams_solve_the_streaming_kernels_batch(count, dims):
