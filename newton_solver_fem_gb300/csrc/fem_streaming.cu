@@ -19,7 +19,8 @@
 //              bit-identical too; removals and topology changes mark their rows
 //   publish    connectivity, poses, materials, masses and flags; contributor
 //              lists rebuilt by a counting sort keyed by SELL entry (ascending
-//              triplet id inside each entry) and the node incidence likewise
+//              triplet id inside each entry, then each id replaced by its
+//              block's place) and the node incidence likewise
 //   assemble   the usual deterministic gather and block-Jacobi inverse
 // Reserved entries without contributors hold exact zeros, so products over the
 // reserved rows equal products over the live entries.  Storage never moves,
@@ -202,7 +203,7 @@ __global__ void contrib_count_kernel(int P, int T, const int* __restrict__ diag_
     }
 }
 
-__global__ void contrib_scatter_kernel(int P, int T, TripletMap map, const int* __restrict__ diag_entry,
+__global__ void contrib_scatter_kernel(int P, int T, const int* __restrict__ diag_entry,
                                        const int* __restrict__ active, const int* __restrict__ slots,
                                        const int* __restrict__ start, int* __restrict__ count,
                                        int* __restrict__ contrib) {
@@ -216,7 +217,16 @@ __global__ void contrib_scatter_kernel(int P, int T, TripletMap map, const int* 
     }
     if (entry < 0) return;
     const int pos = atomicSub(count + entry, 1) - 1;
-    contrib[start[entry] + pos] = (int)map.place(t);  // streaming handles hold no springs or triangles
+    contrib[start[entry] + pos] = (int)t;
+}
+
+// The sorted triplet ids, replaced by the places of their stored blocks (unsigned; streaming handles hold
+// no springs or triangles).  After the sort: places do not ascend with the ids (a group's tets are stored
+// block by block), and they pass 2^31 before the ids do.
+__global__ void contrib_place_kernel(int64_t nsell, TripletMap map, const int* __restrict__ start,
+                                     int* __restrict__ contrib) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < start[nsell]) contrib[i] = (int)map.place(contrib[i]);
 }
 
 // Ascending order inside each segment [start[i], start[i+1]) (insertion sort; segments are short).
@@ -448,9 +458,10 @@ int streaming_update(Handle& h, const FemDesc* d, const float* q, const int* sou
                                                                h.entry_count);
     ok(cudaGetLastError());
     ok(launch_exclusive_scan(h.entry_count, h.sell_cptr, (int)h.nsell, h.scan_part, s));
-    contrib_scatter_kernel<<<blocks_for(nkeys, 256), 256, 0, s>>>(P, T, h.trip_map, h.diag_entry, h.st_active, h.st_slot,
+    contrib_scatter_kernel<<<blocks_for(nkeys, 256), 256, 0, s>>>(P, T, h.diag_entry, h.st_active, h.st_slot,
                                                                  h.sell_cptr, h.entry_count, h.sell_contrib);
     sort_segments_kernel<<<blocks_for(h.nsell, 256), 256, 0, s>>>(h.nsell, h.sell_cptr, h.sell_contrib);
+    contrib_place_kernel<<<blocks_for(nkeys, 256), 256, 0, s>>>(h.nsell, h.trip_map, h.sell_cptr, h.sell_contrib);
     // node incidence of the element-force gather (every corner slot, ascending)
     const int* flat_idx = reinterpret_cast<const int*>(h.tet_idx);
     incidence_count_kernel<<<blocks_for(4 * (int64_t)T, 256), 256, 0, s>>>(T, flat_idx, h.st_active, h.node_count);

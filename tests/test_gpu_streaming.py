@@ -15,7 +15,7 @@ import pytest
 import torch
 from gpu_helpers import DEVICE, tensor, to_np
 
-from newton_solver_fem_gb300 import SolverFEM, _lib, model_from_arrays
+from newton_solver_fem_gb300 import SolverFEM, _lib, model_from_arrays, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -258,3 +258,25 @@ def test_original_capture_replays_after_multiple_edits():
         reference.step(state, expected, None, None, reference.dt)
         np.testing.assert_allclose(to_np(output.particle_q), to_np(expected.particle_q), rtol=2e-5, atol=2e-6)
         np.testing.assert_allclose(to_np(output.particle_qd), to_np(expected.particle_qd), rtol=1e-4, atol=2e-5)
+
+
+@pytest.mark.parametrize("cells,copies", [((5, 4, 3), 1), ((3, 3, 3), 2)])  # 360 and 162 tets: whole and part groups of 32
+def test_update_without_edits_assembles_the_static_handles_bits(cells, copies):
+    """Every sum of the assembly runs in ascending triplet order on both kinds of handle, so on the same
+    elements the matrices and the preconditioners are the same to the bit."""
+    x, tets, mats, mass = scenes.tet_block(*cells, 0.1, (0.0, 0.0, 0.0), 2e4, 0.4, 1000.0)
+    rng = np.random.default_rng(3)
+    n = len(x)
+    x = np.tile(x + rng.uniform(-0.02, 0.02, x.shape), (copies, 1))
+    q = tensor(x + rng.normal(0.0, 5e-3, x.shape))
+
+    def solver():
+        model = model_from_arrays(x, np.tile(mass, copies), tets=tets, tet_materials=mats, device=DEVICE)
+        return SolverFEM(model, dt=1.0 / 120, solver_type="cg", preconditioner_type="block_diag", self_contact_ke=0.0)
+
+    static, streaming = solver(), solver()
+    streaming.prepare_tetrahedral_updates(n)
+    static.refresh_tangent(q)
+    streaming.refresh_topology(q)
+    np.testing.assert_array_equal(streaming.A_bsr.dense(), static.A_bsr.dense())
+    np.testing.assert_array_equal(to_np(streaming._pc_inv_diag), to_np(static._pc_inv_diag))
