@@ -343,8 +343,9 @@ int configure_launch(Handle& h) {
     return FEM_OK;
 }
 
-// The on-chip PCG's plan, tables and records, when the rows fit and the grid is co-resident.
-int plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vector<unsigned>& row_info,
+// The on-chip PCG's plan, tables and records, when the rows fit and the grid is co-resident.  Whatever it
+// cannot have (a launch limit, device memory) leaves the handle without a plan, on the streaming kernel.
+void plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vector<unsigned>& row_info,
                 const std::vector<int>& scol) {
     Handle& h = b.h;
     int dev = 0, sms = 0;
@@ -360,11 +361,13 @@ int plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vect
                               }};
     fem::OnchipPlan plan;
     fem::onchip_plan(h, in, sms, plan);
-    if (plan.grid == 0) return FEM_OK;
+    if (plan.grid == 0) return;
     bool resident = false;
-    cudaError_t e = fem::onchip_allow(plan, sms, &resident);
-    if (e != cudaSuccess) return cuda_status(e, &h);
-    if (!resident) return FEM_OK;
+    if (fem::onchip_allow(plan, sms, &resident) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (!resident) return;
     // one allocation for the tables and one for the records and partials (a small solver's construction
     // is mostly allocations)
     std::vector<unsigned char> blob;
@@ -376,11 +379,19 @@ int plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vect
     };
     const size_t o_slice0 = put(plan.slice0), o_kres = put(plan.kres), o_ptr = put(plan.halo_ptr),
                  o_halo = put(plan.halo), o_lcol = put(plan.lcol), o_team = put(plan.team);
+    const size_t held = h.allocations.size();
     unsigned char* tables = b.upload(blob);
     // records, then the teams' counters, then partials
     const size_t counters = (size_t)h.nscenes * fem::kTeamBarrierBytes / sizeof(float4);
     float4* work = b.alloc<float4>(6 * (size_t)h.P + 8 + counters + 4 * (size_t)plan.grid);
-    if (b.status != FEM_OK) return b.status;
+    if (b.status != FEM_OK) {
+        for (size_t i = held; i < h.allocations.size(); ++i) cudaFree(h.allocations[i]);
+        h.allocations.resize(held);
+        cudaGetLastError();
+        b.status = FEM_OK;
+        h.last_error.clear();
+        return;
+    }
     h.oc_slice0 = reinterpret_cast<int*>(tables + o_slice0);
     h.oc_kres = reinterpret_cast<int2*>(tables + o_kres);
     h.oc_halo_ptr = reinterpret_cast<int*>(tables + o_ptr);
@@ -397,7 +408,6 @@ int plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vect
     h.oc_hybrid = plan.hybrid;
     h.oc_meet = plan.meet;
     h.oc_smem = plan.smem;
-    return FEM_OK;
 }
 
 // Measure each CTA's SpMV-phase speed on 10-iteration solves of a synthetic
@@ -964,7 +974,7 @@ int fem::create_handle(const FemDesc* d, const std::vector<std::vector<int>>* ca
     for (int sl = 0; sl < h.nslices; ++sl)
         for (int l = 0; l < slice_meta[sl].y; ++l) h.host_slice_cost[sl] += row_nnz[slice_meta[sl].x + l] + 4;
     int code = configure_launch(h);
-    if (code == FEM_OK) code = plan_onchip(b, slice_meta, row_info, scol);
+    if (code == FEM_OK) plan_onchip(b, slice_meta, row_info, scol);
     if (code != FEM_OK) {
         g_error = h.last_error;
         fem_destroy(H);

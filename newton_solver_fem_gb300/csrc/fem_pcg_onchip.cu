@@ -41,7 +41,7 @@
 namespace fem {
 namespace {
 
-constexpr int kSmemLimit = 227 * 1024;
+constexpr int kSmemLimit = 227 * 1024 - 1024;  // dynamic: the kernel's static variables take a part of the first 1 KB
 constexpr int kBlockBytes = 16 + 16 + 4 + 2;      // one resident block: values and local column
 constexpr int kColumnBytes = kBlockBytes * kSlice;  // one resident block column of a slice
 constexpr float kPredictFloor = 0.01f;
@@ -837,7 +837,7 @@ void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& pl
                 fits[c] = 0;
                 continue;
             }
-            const int64_t room = (kSmemLimit - fixed_bytes - 1024) / kColumnBytes;
+            const int64_t room = (kSmemLimit - fixed_bytes) / kColumnBytes;
             const int in_regs = regs * oc_parts(warps, ns);  // columns of each slice kept in registers
             auto rest = [&](int sl) {
                 return (int64_t)std::max(0, h.host_slice_ptr[sl + 1] - h.host_slice_ptr[sl] - in_regs);

@@ -304,6 +304,30 @@ def test_onchip_clusters_of_any_size_solve_the_streaming_kernels_system(layers, 
     assert rel_l2(got, run()) < 1e-5
 
 
+@pytest.mark.parametrize("neighbours", [13856, 13917, 13918, 13919, 13920, 13921])
+def test_hub_whose_halo_takes_all_shared_memory(neighbours):
+    """A node joined to 13,856 others by springs leaves its CTA's shared memory no room for a block; from
+    there to 13,921 the halo is within what an SM has but not within what a launch may ask for.  All are
+    created and solved (by the streaming kernel where the halo does not fit); the star's solution is explicit."""
+    from gpu_helpers import make_pair, tensor
+
+    rng = np.random.default_rng(11)
+    P, m, ke, kd, h = 32 + neighbours, 0.5, np.float32(40.0), np.float32(0.01), np.float64(np.float32(1.0 / 600.0))
+    x = rng.uniform(0.0, 1.0, (P, 3))
+    springs = np.stack([np.zeros(neighbours, np.int32), np.arange(32, P, dtype=np.int32)], 1)  # 1..31 stay free
+    model, solver, _ = make_pair(x, np.full(P, m), springs=springs, spring_ke=np.full(neighbours, ke),
+                                 spring_kd=np.full(neighbours, kd), with_oracle=False)
+    rhs = tensor(rng.normal(0.0, 1.0, (P, 3)))
+    y = torch.empty_like(rhs)
+    _lib.check(_lib.load().fem_solve(solver._handle, rhs.data_ptr(), y.data_ptr(), 1e-6, 100, solver._stream()))
+    assert solver.stats()["status"] == 0
+    b, c = to_np(rhs), h * h * ke + h * kd
+    want = b / m
+    want[0] = (b[0] + c * b[32:].sum(0) / (m + c)) / (m + c * neighbours - neighbours * c * c / (m + c))
+    want[32:] = (b[32:] + c * want[0]) / (m + c)
+    assert rel_l2(to_np(y), want) < 1e-5
+
+
 @pytest.mark.parametrize("count,dims", [(2, (2, 3)), (24, (3, 10)), (9, (2, 24)), (152, (2, 5))],
                          ids=lambda v: str(v).replace(" ", ""))
 def test_onchip_teams_solve_the_streaming_kernels_batch(count, dims):
