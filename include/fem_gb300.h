@@ -172,8 +172,9 @@ int fem_set_wait_limit(FemHandle* handle, int64_t nanoseconds);
 
 /* Launch tuning of the persistent PCG kernel (chosen by an autotuner).  Not
  * capturable: a change rebuilds the launch tables. */
-#define FEM_TUNE_SPMV_UNROLL 1       /* block columns in flight per thread: 1, 2 or 4 (default: 4 while the matrix
-                                      * stays in L2 between CG iterations, else 2); read: what is in use */
+#define FEM_TUNE_SPMV_UNROLL 1       /* block columns in flight per thread: 1, 2, 4 or 0 (default, automatic: 4 while
+                                      * the matrix stays in L2 between CG iterations, else 2); read: what is in use.
+                                      * It changes no bit, and does not move solves off the on-chip kernel */
 #define FEM_TUNE_L2_RESIDENT_BYTES 2 /* matrix bytes loaded evict_last (kept in L2 across iterations); -1 = 60% of L2;
                                         -2 (default) = the whole matrix when it fits in 60% of L2, else none */
 #define FEM_TUNE_RESIDENT_SLICES 3   /* read-only: resulting number of L2-resident 32-row slices */
@@ -217,9 +218,9 @@ int fem_set_wait_limit(FemHandle* handle, int64_t nanoseconds);
                                         sets the timeout status that fem_get_stats reports. */
 #define FEM_TUNE_ONCHIP 17           /* the PCG that keeps a CTA's matrix rows in shared memory and its CG vectors in
                                         registers, with one grid reduction per iteration: -1 (default) when the rows
-                                        fit (at most 1024 rows per SM and a scene per SM) and none of the streaming kernel's
-                                        keys above was changed; 0 never; 1 whenever the rows fit (standard recurrence
-                                        and uncalibrated split only) */
+                                        fit (at most 1024 rows per SM and a scene per SM) and no streaming-kernel key
+                                        above but the load depth asks for other than its automatic value; 0 never;
+                                        1 whenever the rows fit (standard recurrence and uncalibrated split only) */
 #define FEM_TUNE_ONCHIP_GRID 18      /* read-only: that kernel's grid, 0 while solves use the streaming kernel */
 int fem_set_tuning(FemHandle* handle, int32_t key, int64_t value);
 int fem_get_tuning(FemHandle* handle, int32_t key, int64_t* value);

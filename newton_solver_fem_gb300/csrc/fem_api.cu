@@ -1343,7 +1343,8 @@ int fem_set_tuning(FemHandle* H, int32_t key, int64_t value) {
     Handle& h = H->h;
     DeviceGuard g(H->device);
     if (key == FEM_TUNE_SPMV_UNROLL) {
-        if (value != 1 && value != 2 && value != 4) return set_error(FEM_ERR_BAD_ARG, "unroll must be 1, 2 or 4");
+        if (value != 0 && value != 1 && value != 2 && value != 4)
+            return set_error(FEM_ERR_BAD_ARG, "unroll must be 0 (automatic), 1, 2 or 4");
         h.spmv_unroll = (int)value;
     } else if (key == FEM_TUNE_L2_RESIDENT_BYTES) {
         if (value < -2) return set_error(FEM_ERR_BAD_ARG, "resident bytes must be >= -2");

@@ -499,12 +499,13 @@ cudaError_t launch_pcg_onchip(Handle& h, float dt, int write_state, float* q_out
                               cudaStream_t s, const float* solve_rhs, float* x_out, float tol, int maxiter,
                               bool solve_warm);
 // Whether this handle's solves run on chip: it has a plan, and no launch option of the streaming
-// kernel was asked for (an explicit request, 1, wins over them; 0 turns it off).
+// kernel was asked for (an explicit request, 1, wins over them; 0 turns it off).  The load depth does not
+// count: it changes no bit of the streaming kernel's results, and its getter reports the depth in use, so a
+// program that saves and restores it would lose this kernel.
 inline bool onchip_in_use(const Handle& h) {
     if (h.oc_grid == 0 || h.onchip == 0 || h.cg_variant != 0 || h.balance != 0) return false;
     return h.onchip == 1 || (h.pcg_threads == 0 && h.grid_cap == 0 && h.resident_pref == -1 && h.compact_cols == -1 &&
-                             h.l2_resident_bytes == -2 && h.spmv_unroll == 0 && h.tail_prefetch == 50 &&
-                             h.split_headroom == 0);
+                             h.l2_resident_bytes == -2 && h.tail_prefetch == 50 && h.split_headroom == 0);
 }
 // Step mode (solve_rhs == nullptr): predictor, normalised PCG from the dv warm start, integration.
 // Solve mode: A x = solve_rhs from zero (projected at fixed rows), x written to x_out.

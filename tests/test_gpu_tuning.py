@@ -141,6 +141,32 @@ def test_automatic_depth_and_row_state_change_no_bit(cap, state, l2_bytes, depth
         np.testing.assert_array_equal(a, b)
 
 
+def test_load_depth_is_saved_restored_and_reset():
+    """Writing back the depth that was read, or the former default of 4, leaves the kernel and every bit of a
+    substep as they are; 0 is automatic again."""
+    sc = scenes.hex_block_64(n=12)
+    model, solver, _ = scene_pair(sc, linear_solver_tolerance=1e-6, linear_solver_maxiter=100, with_oracle=False)
+    lib = _lib.load()
+    put = lambda key, value: _lib.check(lib.fem_set_tuning(solver._handle, key, value))  # noqa: E731
+    for onchip in (-1, 0):
+        put(_lib.FEM_TUNE_ONCHIP, onchip)
+        put(_lib.FEM_TUNE_SPMV_UNROLL, 0)
+        grid, ref = setting(solver, _lib.FEM_TUNE_ONCHIP_GRID), substep(model, solver, sc)
+        assert (grid > 0) == (onchip == -1)
+        for depth in (setting(solver, _lib.FEM_TUNE_SPMV_UNROLL), 4, 2, 1, 0):
+            put(_lib.FEM_TUNE_SPMV_UNROLL, depth)
+            assert setting(solver, _lib.FEM_TUNE_SPMV_UNROLL) == (depth or 4)
+            assert setting(solver, _lib.FEM_TUNE_ONCHIP_GRID) == grid
+            for a, b in zip(substep(model, solver, sc), ref):
+                np.testing.assert_array_equal(a, b)
+    put(_lib.FEM_TUNE_L2_RESIDENT_BYTES, 0)
+    for depth, used in ((0, 2), (4, 4), (0, 2)):
+        put(_lib.FEM_TUNE_SPMV_UNROLL, depth)
+        assert setting(solver, _lib.FEM_TUNE_SPMV_UNROLL) == used
+    for bad in (-1, 3, 8):
+        assert lib.fem_set_tuning(solver._handle, _lib.FEM_TUNE_SPMV_UNROLL, bad) == _lib.FEM_ERR_BAD_ARG
+
+
 def test_column_modes_are_bit_identical_and_report_shared_slots():
     """Column modes only change where a block's column comes from, so substeps agree bit for bit."""
     sc = scenes.hex_block_64(n=12)
