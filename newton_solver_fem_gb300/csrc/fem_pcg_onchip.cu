@@ -665,7 +665,8 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
             a.scene_stats[team.z] = o;
             a.cum_iters[team.z] += st.iters;
             // running max of the relative residual (non-negative floats order like their bit patterns)
-            float rel = st.bb > 0.0f ? (float)sqrt(fmax((double)st.rr, 0.0) / (double)st.bb) : 0.0f;
+            // (a prediction may round below zero; a NaN stays one)
+            float rel = st.bb > 0.0f ? (float)sqrt((st.rr < 0.0f ? 0.0 : (double)st.rr) / (double)st.bb) : 0.0f;
             if (!isfinite(rel)) rel = 1.0e30f;
             atomicMax(reinterpret_cast<int*>(a.resid_max + (step_mode ? 0 : 1)), __float_as_int(rel));
         }

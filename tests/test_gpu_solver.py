@@ -614,3 +614,21 @@ def test_matrix_export_writes_the_assembled_blocks_and_nothing_else(star):
     offsets = torch.full_like(whole.offsets, -1)
     _lib.check(solver._lib.fem_export_bsr(solver._handle, offsets.data_ptr(), None, None, solver._stream()))
     assert torch.equal(offsets, whole.offsets)
+
+
+@pytest.mark.parametrize("onchip", [0, -1])
+@pytest.mark.parametrize("cells", [(2, 2, 2), (13, 12, 11)])  # one CTA, and a grid
+def test_a_residual_that_is_no_number_is_reported_and_refused(onchip, cells):
+    """A NaN in the start makes the residual NaN over a finite right-hand side: the largest relative residual
+    reads 1e30, the differentiable mode's check raises, and the status says non-finite."""
+    x, hexes, mats, mass = scenes.hex_block(*cells, 0.01, (0.0, 0.0, 0.0), 2e5, 0.4, 1000.0)
+    model, solver, _ = make_pair(x, mass, hexes=hexes, hex_materials=mats, with_oracle=False)
+    _lib.check(_lib.load().fem_set_tuning(solver._handle, _lib.FEM_TUNE_ONCHIP, onchip))
+    solver.velocity_increment[len(x) // 2, 1] = float("nan")
+    solver.step(model.state(), model.state(), None, None, solver.dt)
+    with pytest.raises(RuntimeError, match="did not converge"):
+        solver.check()
+    assert solver.last_differentiation_residuals["forward_relative_residual"] == np.float32(1e30)
+    with pytest.raises(_lib.FemError) as err:
+        solver.stats()
+    assert err.value.code == _lib.FEM_ERR_NON_FINITE
