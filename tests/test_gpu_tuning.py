@@ -330,6 +330,48 @@ def test_onchip_clusters_of_any_size_solve_the_streaming_kernels_system(layers, 
     assert rel_l2(got, run()) < 1e-5
 
 
+@pytest.mark.parametrize("element,cells", [("hex", (1, 1, 1)), ("tet", (1, 1, 1)), ("hex", (2, 2, 2)), ("hex", (3, 2, 2)),
+                                           ("hex", (3, 3, 3)), ("tet", (40, 1, 1))])
+def test_onchip_iterates_of_the_smallest_bodies_are_as_exact_as_the_streaming_kernels(element, cells):
+    """Bodies that one CTA solves converge in steep last steps, where rounding in CG's scalars shows most.  After
+    the steps that 64-bit CG takes to 1e-4, the mean distance from its iterates over 24 right-hand sides is at
+    most half again the streaming kernel's (the same sums in another order, so samples of one spread)."""
+    from gpu_helpers import make_pair
+
+    block = scenes.tet_block if element == "tet" else scenes.hex_block
+    x, el, mats, mass = block(*cells, 0.01, (0.0, 0.0, 0.0), 3e5, 0.4, 1000.0)
+    fixed = np.nonzero(np.isclose(x[:, 0], 0.0))[0].astype(np.int32)
+    elements = {"tets": el, "tet_materials": mats} if element == "tet" else {"hexes": el, "hex_materials": mats}
+    model, solver, _ = make_pair(x, mass, fixed=fixed, with_oracle=False, **elements)
+    P, lib = len(x), _lib.load()
+    keep = np.ones((P, 3))
+    keep[fixed] = 0.0
+    keep = keep.ravel()
+    A, minv = solver.A_bsr.dense().astype(np.float64), to_np(solver._pc_inv_diag).reshape(P, 3, 3)
+    precondition = lambda r: np.einsum("nij,nj->ni", minv, r.reshape(P, 3)).ravel()  # noqa: E731
+    off = {0: [], -1: []}
+    for seed in range(24):
+        b = (np.random.default_rng(seed).normal(0.0, 1.0, x.shape) * mass[:, None]).astype(np.float32)
+        b[fixed] = 0.0
+        rhs = torch.tensor(b, device="cuda")
+        r = b.astype(np.float64).ravel()
+        want, z, stop, steps = np.zeros(3 * P), precondition(r), 1e-8 * (r @ r), 0
+        p, rz = z, r @ z
+        while r @ r > stop:
+            y = keep * (A @ p)
+            alpha = rz / (p @ y)
+            want, r = want + alpha * p, r - alpha * y
+            z = precondition(r)
+            p, rz = z + (r @ z) / rz * p, r @ z
+            steps += 1
+        for onchip in (0, -1):
+            _lib.check(lib.fem_set_tuning(solver._handle, _lib.FEM_TUNE_ONCHIP, onchip))
+            y = torch.empty_like(rhs)
+            _lib.check(lib.fem_solve(solver._handle, rhs.data_ptr(), y.data_ptr(), 1e-30, steps, solver._stream()))
+            off[onchip].append(rel_l2(to_np(y), want))
+    assert np.mean(off[-1]) < 1.5 * np.mean(off[0])
+
+
 @pytest.mark.parametrize("neighbours", [13856, 13917, 13918, 13919, 13920, 13921])
 def test_hub_whose_halo_takes_all_shared_memory(neighbours):
     """A node joined to 13,856 others by springs leaves its CTA's shared memory no room for a block; from
