@@ -46,6 +46,11 @@ constexpr int kSmemLimit = 227 * 1024 - 1024;  // dynamic: the kernel's static v
 constexpr int kBlockBytes = 16 + 16 + 4 + 2;      // one resident block: values and local column
 constexpr int kColumnBytes = kBlockBytes * kSlice;  // one resident block column of a slice
 constexpr float kPredictFloor = 0.01f;
+// A predicted rr1 carries the sums' rounding times at most (2 / sqrt(rr1 / rr) + 1)^2: 441 at kPredictFloor, 15 at
+// kStopFloor.  So the stop is decided by the sum itself when the prediction is within kStopMargin of the
+// threshold, and the residual that a solve reports is the sum itself unless its last step reduced it by less
+// than that (most do: a reduction at every stop cost 1.5 us in a cluster, 3.5 in a grid).
+constexpr float kStopMargin = 1.01f, kStopFloor = 0.5f;
 
 // Scalars of the solve, formed by one thread from float totals (float32, like the reference's dot
 // products; FP64 is far slower here and sits on every iteration's critical path: a quotient of two
@@ -667,7 +672,10 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
                 st.rr = rr1;
                 st.rz = rz;
                 st.iters += 1;
-                st.again = rz1 < kPredictFloor * rz || rr1 < kPredictFloor * rr;
+                const bool below = rr1 <= kStopMargin * st.floor_rr;
+                st.again = rz1 < kPredictFloor * rz || rr1 < kPredictFloor * rr ||
+                           ((below || st.iters >= a.maxiter) && rr1 < kStopFloor * rr) ||
+                           (below && kStopMargin * rr1 > st.floor_rr);
                 st.active = (rr1 > st.floor_rr) && (st.iters < a.maxiter);
                 if (!isfinite(rr1)) {
                     st.active = 0;
@@ -676,7 +684,7 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
                 }
             });
         }
-        if (ok && st.again) {  // the predictions cancelled: the sums themselves
+        if (ok && st.again) {  // the predictions cancelled too far for what they decide: the sums themselves
             const float a1 = st.alpha;
             const float3 r1 = f3(fmaf(-a1, s.x, r.x), fmaf(-a1, s.y, r.y), fmaf(-a1, s.z, r.z));
             float v[8] = {dot3(r1, precondition(r1)), dot3(r1, r1), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};

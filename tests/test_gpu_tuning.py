@@ -372,6 +372,41 @@ def test_onchip_iterates_of_the_smallest_bodies_are_as_exact_as_the_streaming_ke
     assert np.mean(off[-1]) < 1.5 * np.mean(off[0])
 
 
+@pytest.mark.parametrize("tolerance,maxiter", [(0.3, 50), (1e-4, 1)])  # ends by the threshold, and by the cap
+@pytest.mark.parametrize("cells", [(9, 9, 9), (16, 15, 14)])  # a cluster, a grid
+def test_onchip_reports_the_residual_after_a_steep_last_step(cells, tolerance, maxiter):
+    """A right-hand side that is a generalised eigenvector of A and the preconditioner plus a fifth of noise: one
+    step cuts ||r||^2 to 1 to 10 percent.  The reported residual is the 64-bit ||b - A x|| / ||b|| up to the rounding
+    of a float sum, on the mean of 16 noises less than one float32 unit; a prediction is off by the cancelled factor."""
+    sp = pytest.importorskip("scipy.sparse")
+    from gpu_helpers import make_pair
+    from scipy.sparse.linalg import eigsh
+
+    x, hexes, mats, mass = scenes.hex_block(*cells, 0.01, (0.0, 0.0, 0.0), 2e5, 0.4, 1000.0)
+    model, solver, _ = make_pair(x, mass, hexes=hexes, hex_materials=mats, with_oracle=False)
+    P, bsr = len(x), solver.A_bsr
+    at = (bsr.columns.cpu().numpy(), bsr.offsets.cpu().numpy())
+    A = sp.bsr_matrix((to_np(bsr.values), *at), shape=(3 * P, 3 * P)).tocsr()
+    minv = to_np(solver._pc_inv_diag).reshape(P, 3, 3)
+    rows = (np.arange(P), np.arange(P + 1))
+    M = sp.bsr_matrix((np.linalg.inv(minv), *rows), shape=A.shape).tocsc()
+    v = eigsh(A, k=1, M=M, Minv=sp.bsr_matrix((minv, *rows), shape=A.shape).tocsc(), which="LM", v0=np.ones(3 * P))[1][:, 0]
+    assert setting(solver, _lib.FEM_TUNE_ONCHIP_GRID) > 1
+    off = []
+    for seed in range(16):
+        b, noise = A @ v, (np.random.default_rng(seed).normal(0.0, 1.0, x.shape) * mass[:, None]).ravel()
+        b = (b / np.linalg.norm(b) + 0.2 * noise / np.linalg.norm(noise)).astype(np.float32)
+        rhs = torch.tensor(b.reshape(P, 3), device="cuda")
+        y = torch.empty_like(rhs)
+        _lib.check(_lib.load().fem_solve(solver._handle, rhs.data_ptr(), y.data_ptr(), tolerance, maxiter, solver._stream()))
+        b, got = b.astype(np.float64), solver.stats()
+        true = np.linalg.norm(b - A @ to_np(y).ravel()) / np.linalg.norm(b)
+        assert got["max_iterations"] == 1 and 0.1 < true < 0.33
+        assert got["unconverged_scenes"] == (maxiter == 1)
+        off.append(abs(got["max_relative_residual"] / true - 1.0))
+    assert np.mean(off) < 2.0 ** -23
+
+
 @pytest.mark.parametrize("neighbours", [13856, 13917, 13918, 13919, 13920, 13921])
 def test_hub_whose_halo_takes_all_shared_memory(neighbours):
     """A node joined to 13,856 others by springs leaves its CTA's shared memory no room for a block; from
