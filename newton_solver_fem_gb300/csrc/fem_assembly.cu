@@ -184,8 +184,9 @@ __global__ void __launch_bounds__(kExportThreads) export_bsr_kernel(const Export
     if (threadIdx.x >= 64 && tail < n) out[tail] = t[tail];
 }
 
-// The same for slices too wide for that: a warp takes kExportColumns block columns of a slice
-// (blockIdx.y) and writes each row's run of them (62 us for the 3.05 million blocks).
+// The same for slices too wide for that: a warp takes kExportColumns block columns of a slice at a time
+// (blockIdx.y, and on by gridDim.y, which ends at 65,535) and writes each row's run of them (62 us for the 3.05
+// million blocks).
 constexpr int kExportColumns = 8, kExportWarps = 4;
 constexpr int kExportRow = 9 * kExportColumns + 1;  // padded: the 32 rows of a column in distinct banks
 
@@ -195,30 +196,32 @@ __global__ void __launch_bounds__(32 * kExportWarps) export_columns_kernel(
     const float* __restrict__ valC, float* __restrict__ out) {
     __shared__ float tile[kExportWarps][32 * kExportRow];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int sl = blockIdx.x * kExportWarps + w, k0 = blockIdx.y * kExportColumns;
+    const int sl = blockIdx.x * kExportWarps + w;
     if (sl >= nslices) return;  // the whole warp
-    const int base = slice_ptr[sl];
-    if (base + k0 >= slice_ptr[sl + 1]) return;
+    const int base = slice_ptr[sl], width = slice_ptr[sl + 1] - base;
     const int2 m = meta[sl];
     const bool live = lane < m.y;
     const int len = live ? (int)(row_info[m.x + lane] & ~kFixedBit) : 0;
     const int start = live ? offsets[m.x + lane] : 0;
     float* t = tile[w];
+    for (int k0 = blockIdx.y * kExportColumns; k0 < width; k0 += gridDim.y * kExportColumns) {
 #pragma unroll
-    for (int u = 0; u < kExportColumns; ++u)
-        if (k0 + u < len) {
-            const size_t e = (size_t)(base + k0 + u) * kSlice + lane;
-            const float4 a = __ldg(valA + e), b = __ldg(valB + e);
-            float* o = t + lane * kExportRow + 9 * u;
-            o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-            o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-            o[8] = __ldg(valC + e);
+        for (int u = 0; u < kExportColumns; ++u)
+            if (k0 + u < len) {
+                const size_t e = (size_t)(base + k0 + u) * kSlice + lane;
+                const float4 a = __ldg(valA + e), b = __ldg(valB + e);
+                float* o = t + lane * kExportRow + 9 * u;
+                o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+                o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+                o[8] = __ldg(valC + e);
+            }
+        __syncwarp();
+        for (int r = 0; r < m.y; ++r) {
+            const int n = 9 * min(kExportColumns, __shfl_sync(0xffffffffu, len, r) - k0);
+            float* o = out + 9 * ((size_t)__shfl_sync(0xffffffffu, start, r) + k0);
+            for (int i = lane; i < n; i += 32) o[i] = t[r * kExportRow + i];
         }
-    __syncwarp();
-    for (int r = 0; r < m.y; ++r) {
-        const int n = 9 * min(kExportColumns, __shfl_sync(0xffffffffu, len, r) - k0);
-        float* o = out + 9 * ((size_t)__shfl_sync(0xffffffffu, start, r) + k0);
-        for (int i = lane; i < n; i += 32) o[i] = t[r * kExportRow + i];
+        __syncwarp();  // the tile is read before it is written again
     }
 }
 
@@ -262,7 +265,8 @@ cudaError_t launch_export_bsr(Handle& h, int* offsets, int* columns, float* valu
         export_bsr_kernel<<<a.pattern_blocks + slices, kExportThreads, bytes, s>>>(a);
     }
     if (values != nullptr && !narrow)
-        export_columns_kernel<<<dim3(blocks_for(h.nslices, kExportWarps), blocks_for(h.slice_width, kExportColumns)),
+        export_columns_kernel<<<dim3(blocks_for(h.nslices, kExportWarps),
+                                     std::min(65535, blocks_for(h.slice_width, kExportColumns))),
                                 32 * kExportWarps, 0, s>>>(h.nslices, h.slice_ptr, h.slice_meta, h.row_info,
                                                            h.bsr_offsets, h.valA, h.valB, h.valC, values);
     return cudaGetLastError();

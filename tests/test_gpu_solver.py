@@ -616,6 +616,27 @@ def test_matrix_export_writes_the_assembled_blocks_and_nothing_else(star):
     assert torch.equal(offsets, whole.offsets)
 
 
+def test_matrix_export_of_a_row_wider_than_a_grid():
+    """A hub with 524,288 spring neighbours: its row has more groups of eight block columns than a launch has
+    rows of blocks (65,535).  The matrix of a star is explicit."""
+    n, m, ke, kd, h = 524_288, 0.5, np.float32(40.0), np.float32(0.01), np.float64(np.float32(1.0 / 600.0))
+    x = np.random.default_rng(12).uniform(0.0, 1.0, (n + 1, 3))
+    springs = np.stack([np.zeros(n, np.int32), np.arange(1, n + 1, dtype=np.int32)], 1)
+    model, solver, _ = make_pair(x, np.full(n + 1, m), springs=springs, spring_ke=np.full(n, ke),
+                                 spring_kd=np.full(n, kd), with_oracle=False)
+    A, c = solver.A_bsr, h * h * ke + h * kd
+    np.testing.assert_array_equal(A.offsets.cpu().numpy(), np.concatenate([[0], n + 1 + 2 * np.arange(n + 1)]))
+    np.testing.assert_array_equal(A.columns[: n + 1].cpu().numpy(), np.arange(n + 1))
+    values = to_np(A.values)
+    hub, leaves = values[: n + 1], values[n + 1:].reshape(n, 2, 3, 3)
+    eye = np.eye(3)
+    summed = np.add.accumulate(np.concatenate([[m], np.full(n, c)]).astype(np.float32))[-1]  # in order, in float32
+    np.testing.assert_allclose(hub[0], eye * summed, rtol=1e-3, atol=0.0)
+    np.testing.assert_allclose(hub[1:], np.broadcast_to(-c * eye, (n, 3, 3)), rtol=1e-6, atol=0.0)
+    np.testing.assert_allclose(leaves[:, 0], np.broadcast_to(-c * eye, (n, 3, 3)), rtol=1e-6, atol=0.0)
+    np.testing.assert_allclose(leaves[:, 1], np.broadcast_to((m + c) * eye, (n, 3, 3)), rtol=1e-6, atol=0.0)
+
+
 @pytest.mark.parametrize("onchip", [0, -1])
 @pytest.mark.parametrize("cells", [(2, 2, 2), (13, 12, 11)])  # one CTA, and a grid
 def test_a_residual_that_is_no_number_is_reported_and_refused(onchip, cells):
