@@ -218,7 +218,8 @@ int fem_set_wait_limit(FemHandle* handle, int64_t nanoseconds);
                                         sets the timeout status that fem_get_stats reports. */
 #define FEM_TUNE_ONCHIP 17           /* the PCG that keeps a CTA's matrix rows in shared memory and its CG vectors in
                                         registers, with one grid reduction per iteration: -1 (default) when the rows
-                                        fit (at most 1024 rows per SM and a scene per SM) and no streaming-kernel key
+                                        fit (at most 1024 rows per SM and a scene per SM), the node numbering is local
+                                        enough, what is left in L2 stays there, and no streaming-kernel key
                                         above but the load depth asks for other than its automatic value; 0 never;
                                         1 whenever the rows fit (standard recurrence and uncalibrated split only) */
 #define FEM_TUNE_ONCHIP_GRID 18      /* read-only: that kernel's grid, 0 while solves use the streaming kernel */

@@ -348,9 +348,10 @@ int configure_launch(Handle& h) {
 void plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vector<unsigned>& row_info,
                 const std::vector<int>& scol) {
     Handle& h = b.h;
-    int dev = 0, sms = 0;
+    int dev = 0, sms = 0, l2 = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
     const fem::OnchipInput in{scol, slice_meta, row_info,
                               [&](int grid) {
                                   return split_slices(h.host_slice_cost, std::vector<double>(grid, 1.0),
@@ -360,7 +361,7 @@ void plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vec
                                   parallel_for(n, fn, h.nsell < 200000 ? n + 1 : 2);  // threads only for much work
                               }};
     fem::OnchipPlan plan;
-    fem::onchip_plan(h, in, sms, plan);
+    fem::onchip_plan(h, in, sms, l2, plan);
     if (plan.grid == 0) return;
     bool resident = false;
     if (fem::onchip_allow(plan, sms, &resident) != cudaSuccess) {
@@ -404,6 +405,7 @@ void plan_onchip(Builder& b, const std::vector<int2>& slice_meta, const std::vec
     h.oc_barrier = reinterpret_cast<unsigned*>(line);
     h.oc_part = reinterpret_cast<float*>(line + counters);
     h.oc_grid = plan.grid;
+    h.oc_faster = plan.faster;
     h.oc_threads = plan.threads;
     h.oc_hybrid = plan.hybrid;
     h.oc_meet = plan.meet;

@@ -375,6 +375,7 @@ struct Handle {
     bool dv_owned = true;
     // on-chip PCG (fem_pcg_onchip.cu): launch shape and tables, oc_grid 0 when the rows do not fit
     int oc_grid = 0, oc_threads = 0, oc_hybrid = 0, oc_meet = 0;
+    bool oc_faster = false;  // than the streaming kernel, by the plan's halo and what it leaves to L2
     size_t oc_smem = 0;
     int* oc_slice0 = nullptr;
     int4* oc_team = nullptr;
@@ -487,24 +488,25 @@ struct OnchipInput {  // host copies of the SELL layout, and helpers
 };
 struct OnchipPlan {
     int grid = 0, threads = 0, hybrid = 0, meet = 0;
+    bool faster = false;
     size_t smem = 0;
     std::vector<int> slice0, halo_ptr, halo;
     std::vector<int2> kres;
     std::vector<int4> team;
     std::vector<unsigned short> lcol;
 };
-void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& plan);
+void onchip_plan(const Handle& h, const OnchipInput& in, int sms, int64_t l2_bytes, OnchipPlan& plan);
 cudaError_t onchip_allow(const OnchipPlan& plan, int sms, bool* resident);
 cudaError_t launch_pcg_onchip(Handle& h, float dt, int write_state, float* q_out, float* v_out, float* f_ws,
                               cudaStream_t s, const float* solve_rhs, float* x_out, float tol, int maxiter,
                               bool solve_warm);
-// Whether this handle's solves run on chip: it has a plan, and no launch option of the streaming
-// kernel was asked for (an explicit request, 1, wins over them; 0 turns it off).  The load depth does not
+// Whether this handle's solves run on chip: it has a plan that is the faster one, and no launch option of the
+// streaming kernel was asked for (an explicit request, 1, wins over them; 0 turns it off).  The load depth does not
 // count: it changes no bit of the streaming kernel's results, and its getter reports the depth in use, so a
 // program that saves and restores it would lose this kernel.
 inline bool onchip_in_use(const Handle& h) {
     if (h.oc_grid == 0 || h.onchip == 0 || h.cg_variant != 0 || h.balance != 0) return false;
-    return h.onchip == 1 || (h.pcg_threads == 0 && h.grid_cap == 0 && h.resident_pref == -1 && h.compact_cols == -1 &&
+    return h.onchip == 1 || (h.oc_faster && h.pcg_threads == 0 && h.grid_cap == 0 && h.resident_pref == -1 && h.compact_cols == -1 &&
                              h.l2_resident_bytes == -2 && h.tail_prefetch == 50 && h.split_headroom == 0);
 }
 // Step mode (solve_rhs == nullptr): predictor, normalised PCG from the dv warm start, integration.

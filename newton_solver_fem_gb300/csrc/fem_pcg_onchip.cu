@@ -757,6 +757,17 @@ constexpr int kOcRegs = 4, kOcWideWarps = 16;
 //   a cluster of 16 reaches a grid's 3.4 near 2,000 columns (Hex8 74 slices, 1,998 columns: 3.22 and
 //   3.39; Tet4 106 slices, 1,590: 3.16 and 3.34; Hex8 106 slices, 2,862: 3.85 and 3.47).
 constexpr int64_t kAloneColumns = 128, kClusterColumns = 2000;
+// Where the streaming kernel is the faster one although the rows fit (us per iteration, streaming and on chip):
+//   a CTA reads a 48-byte record for every halo column, so a numbering without locality costs it more than the
+//   streaming kernel, whose gathers are as many blocks as before.  Tet4 with nodes numbered at random: 42,875 nodes
+//   (3,746 halo and 132 block columns a CTA) 12.3 and 9.5, 50,653 (4,589, 156) 12.5 and 14.0, 68,921 (6,207, 213) 13.5
+//   and 17.7; Hex8 32,768 (5,169, 182) 14.8 and 13.8, 68,921 (10,964, 383) 18.0 and 25.7; numbers off by about 3,000
+//   places: Tet4 68,921 (4,915, 213) 14.0 and 14.3, 148,877 (8,454, 459) 22.8 and 23.8, Hex8 68,921 (7,414, 383) 18.1
+//   and 18.2.  The line through the crossings is kHaloBase + kHaloPerColumn x block columns;
+//   the columns that are not on chip are read from L2 until they no longer stay there: Hex8 117,649 nodes (89 MB)
+//   27.4 and 21.5, 125,000 (97 MB) 27.7 and 27.5, 132,651 (105 MB) 29.3 and 29.6, 140,608 (113 MB) 30.3 and 32.8.
+constexpr int kHaloBase = 3000, kHaloPerColumn = 10;
+constexpr double kL2Share = 0.7;
 template <Meet kMeet>
 OcKernel oc_kernel_for(int threads, bool hybrid) {
     if (threads <= 32 * kOcWideWarps)
@@ -821,7 +832,7 @@ static void plan_teams(const Handle& h, int sms, OnchipPlan& plan) {
 
 // Lays a handle out for the on-chip kernel: the CTAs' slices, their halo lists and local columns and
 // the resident share of the columns.  Leaves plan.grid 0 when the rows do not fit.
-void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& plan) {
+void onchip_plan(const Handle& h, const OnchipInput& in, int sms, int64_t l2_bytes, OnchipPlan& plan) {
     plan = OnchipPlan{};
     if (h.nslices == 0 || h.nscenes > sms) return;
     int width = 0;
@@ -862,7 +873,8 @@ void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& pl
     plan.halo_ptr.assign(grid + 1, 0);
     std::vector<std::vector<int>> halos(grid);
     std::vector<char> fits(grid, 1);
-    std::vector<int> bytes(grid, 0), partial(grid, 0);
+    std::vector<int> bytes(grid, 0), partial(grid, 0), slow(grid, 0);
+    std::vector<int64_t> streamed(grid, 0);  // block columns read from L2 in every iteration
     in.parallel(grid, [&](int64_t lo, int64_t hi) {
         std::vector<int> local(h.P, -1);
         for (int64_t c = lo; c < hi; ++c) {
@@ -914,15 +926,23 @@ void onchip_plan(const Handle& h, const OnchipInput& in, int sms, OnchipPlan& pl
                 at += k;
             }
             if (total > room) partial[c] = 1;
+            streamed[c] = total - at;
+            const int64_t stored = h.host_slice_ptr[s1] - h.host_slice_ptr[s0];
+            slow[c] = (int64_t)halo.size() > kHaloBase + kHaloPerColumn * stored;
             bytes[c] = fixed_bytes + (int)at * kColumnBytes;
         }
     });
+    plan.faster = true;
+    int64_t from_l2 = 0;
     for (int c = 0; c < grid; ++c) {
         if (!fits[c]) return;
+        if (slow[c]) plan.faster = false;
+        from_l2 += streamed[c] * kColumnBytes;
         plan.halo_ptr[c + 1] = plan.halo_ptr[c] + (int)halos[c].size();
         plan.smem = std::max(plan.smem, (size_t)bytes[c]);
         plan.hybrid = plan.hybrid || partial[c];
     }
+    if ((double)from_l2 > kL2Share * (double)l2_bytes) plan.faster = false;
     plan.halo.reserve(plan.halo_ptr[grid]);
     for (auto& v : halos) plan.halo.insert(plan.halo.end(), v.begin(), v.end());
     plan.threads = 32 * warps;

@@ -407,6 +407,40 @@ def test_onchip_reports_the_residual_after_a_steep_last_step(cells, tolerance, m
     assert np.mean(off) < 2.0 ** -23
 
 
+@pytest.mark.parametrize("element,cells,spread,onchip", [
+    ("hex", (48, 48, 48), 0, True), ("hex", (51, 51, 51), 0, False), ("tet", (52, 52, 52), 0, True),
+    ("tet", (34, 34, 34), -1, True), ("tet", (38, 38, 38), -1, False), ("hex", (33, 33, 33), -1, False),
+    ("tet", (46, 46, 46), 300, True), ("tet", (46, 46, 46), 10000, False)])
+def test_onchip_is_left_where_the_streaming_kernel_is_faster(element, cells, spread, onchip):
+    """Large bodies whose columns do not stay in L2 and numberings without locality (a spread of -1 is random)
+    stream by default; asked for, the on-chip kernel still solves the same system to the variants' bound."""
+    from gpu_helpers import make_pair
+
+    block = scenes.tet_block if element == "tet" else scenes.hex_block
+    x, el, mats, mass = block(*cells, 0.01, (0.0, 0.0, 0.0), 2e5, 0.4, 1000.0)
+    P, rng = len(x), np.random.default_rng(1)
+    order = np.arange(P) if spread == 0 else np.argsort(np.arange(P) + rng.normal(0.0, spread if spread > 0 else 100.0 * P, P))
+    place = np.empty(P, np.int64)
+    place[order] = np.arange(P)
+    x, mass, el = x[order], mass[order], place[el].astype(np.int32)
+    elements = {"tets": el, "tet_materials": mats} if element == "tet" else {"hexes": el, "hex_materials": mats}
+    model, solver, _ = make_pair(x, mass, with_oracle=False, **elements)
+    lib = _lib.load()
+    rhs = torch.tensor((rng.normal(0.0, 1.0, x.shape) * mass[:, None]).astype(np.float32), device="cuda")
+
+    def solve(mode):
+        _lib.check(lib.fem_set_tuning(solver._handle, _lib.FEM_TUNE_ONCHIP, mode))
+        y = torch.empty_like(rhs)
+        _lib.check(lib.fem_solve(solver._handle, rhs.data_ptr(), y.data_ptr(), 1e-6, 200, solver._stream()))
+        assert solver.stats()["status"] == 0
+        return to_np(y), setting(solver, _lib.FEM_TUNE_ONCHIP_GRID) > 0
+
+    (auto, used), (asked, forced), (streamed, off) = solve(-1), solve(1), solve(0)
+    assert used == onchip and forced and not off
+    np.testing.assert_array_equal(auto, asked if onchip else streamed)
+    assert rel_l2(asked, streamed) < 1e-5
+
+
 @pytest.mark.parametrize("neighbours", [13856, 13917, 13918, 13919, 13920, 13921])
 def test_hub_whose_halo_takes_all_shared_memory(neighbours):
     """A node joined to 13,856 others by springs leaves its CTA's shared memory no room for a block; from
