@@ -540,6 +540,41 @@ def test_barrier_wait_limit_reports_timeout_and_recovers():
     assert np.isfinite(to_np(s1.particle_q)).all()
 
 
+@pytest.mark.parametrize("onchip", [0, -1], ids=["streaming", "onchip"])
+@pytest.mark.parametrize("batch", [False, True], ids=["grid", "teams"])
+def test_every_barrier_recovers_from_a_wait_that_ran_out(onchip, batch):
+    """The streaming kernel's grid barrier, the on-chip grid's and the on-chip teams' (each with its own counter,
+    which its last CTA clears): a limit of zero ends the solve with a status, and the solves after a reset give
+    the bits of a handle that never timed out."""
+    sc = scenes.batched_scenes(count=9, seed=7, dims=(2, 24)) if batch else scenes.hex_block_64(n=24)
+    lib = _lib.load()
+
+    def fresh():
+        model, solver, _ = scene_pair(sc, with_oracle=False)
+        _lib.check(lib.fem_set_tuning(solver._handle, _lib.FEM_TUNE_ONCHIP, onchip))
+        return model, solver
+
+    def substeps(model, solver):
+        a, b = model.state(), model.state()
+        for _ in range(3):
+            solver.step(a, b, None, None, sc.dt)
+            a, b = b, a
+        assert solver.stats()["status"] == 0
+        return to_np(a.particle_q), to_np(solver.velocity_increment)
+
+    model, solver = fresh()
+    _lib.check(lib.fem_set_wait_limit(solver._handle, 0))
+    for _ in range(2):
+        solver.step(model.state(), model.state(), None, None, sc.dt)
+    with pytest.raises(_lib.FemError) as err:
+        solver.stats()
+    assert err.value.code == _lib.FEM_ERR_TIMEOUT
+    _lib.check(lib.fem_set_wait_limit(solver._handle, 2_000_000_000))
+    solver.reset()
+    for got, want in zip(substeps(model, solver), substeps(*fresh())):
+        np.testing.assert_array_equal(got, want)
+
+
 def test_large_hex_block_true_residual_property():
     """Full-size Hex8 64^3 block: one substep's true relative residual <= tol, re-checked in float64."""
     sp = pytest.importorskip("scipy.sparse")
