@@ -332,13 +332,17 @@ def batched_measurement(device: str, steps: int, warmup: int) -> dict:
 
 
 def launch_shape(solver) -> dict:
-    """The PCG launch configuration a handle uses (the tuning getters)."""
+    """The PCG launch configuration a handle uses (the tuning getters); the streaming kernel's only where that runs."""
     import ctypes
 
     from newton_solver_fem_gb300 import _lib
 
     lib = _lib.load()
-    out = {}
+    onchip = ctypes.c_int64()
+    _lib.check(lib.fem_get_tuning(solver._handle, _lib.FEM_TUNE_ONCHIP_GRID, ctypes.byref(onchip)))
+    if onchip.value > 0:
+        return {"kernel": "onchip_pcg_kernel", "pcg_ctas": int(onchip.value)}
+    out = {"kernel": "pcg_kernel"}
     for name, key in (("pcg_ctas", _lib.FEM_TUNE_GRID), ("cta_threads", _lib.FEM_TUNE_CTA_THREADS),
                       ("column_mode", _lib.FEM_TUNE_COMPACT_COLUMNS), ("l2_resident_slices", _lib.FEM_TUNE_RESIDENT_SLICES),
                       ("resident_row_state", _lib.FEM_TUNE_RESIDENT_STATE), ("spmv_unroll", _lib.FEM_TUNE_SPMV_UNROLL),
@@ -439,7 +443,7 @@ def tet_measurement(device: str, steps: int, warmup: int) -> dict:
             "ms_per_frame": ms, "value": 3 * P * sc.substeps / (ms / 1e3), "unit": UNIT,
             "mean_cg_iterations": iters, "cg_iterations_timed": iters * steps * sc.substeps,
             "launch": shape, "l2_resident_matrix_bytes": 40 * solver.matrix_info()["stored_blocks"]
-            if shape["l2_resident_slices"] else 0, "finite": finite}
+            if shape.get("l2_resident_slices") else 0, "finite": finite}
 
 
 def adjoint_measurement(device: str, repeats: int) -> dict:
@@ -813,8 +817,9 @@ def run_gb300(args) -> None:
                        "cg_maxiter": sc.maxiter, "preconditioner": "block_diag", "parallelism": "replicas",
                        "nnzb": info["nnzb"], "mean_cg_iterations": timed_iterations,
                        "frames": f"0..{args.steps - 1} from the initial state (reset after warm-up)",
-                       "autotuned": {"choice": {k: tuned[k] for k in ("unroll", "threads", "cg_variant", "grid")},
+                       "autotuned": {"choice": {k: tuned[k] for k in ("unroll", "threads", "cg_variant", "grid", "onchip_grid")},
                                      "us_per_cg_iteration": {
+                                         f"onchip_{r['onchip_grid']}" if r["onchip_grid"] else
                                          f"u{r['unroll']}_t{r['threads']}_v{r['cg_variant']}":
                                              round(r["us_per_iteration"], 2) for r in tuned["candidates"]}},
                        "launch": launch_shape(solver),

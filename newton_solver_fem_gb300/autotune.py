@@ -59,8 +59,7 @@ AXES = {
     "resident_bytes": _lib.FEM_TUNE_L2_RESIDENT_BYTES,
     "onchip": _lib.FEM_TUNE_ONCHIP,
 }
-# the on-chip kernel (the streaming kernel's first shape again where the rows do not fit), then the
-# streaming kernel: every staging depth at every CTA size with the standard recurrence, plus the
+# the on-chip kernel (passed over where the handle has no plan for it), then the streaming kernel: every staging depth at every CTA size with the standard recurrence, plus the
 # single-reduction recurrence at the default shape
 DEFAULT_CANDIDATES = [dict(unroll=4, threads=1024, cg_variant=0, resident_bytes=-2, onchip=1)] + \
                      [dict(unroll=u, threads=t, cg_variant=0, resident_bytes=-2, onchip=0)
@@ -86,7 +85,8 @@ def apply(solver, choice: dict) -> None:
 def current(solver) -> dict:
     lib = _lib.load()
     out = {}
-    for name, key in (*AXES.items(), ("resident_slices", _lib.FEM_TUNE_RESIDENT_SLICES), ("grid", _lib.FEM_TUNE_GRID)):
+    for name, key in (*AXES.items(), ("resident_slices", _lib.FEM_TUNE_RESIDENT_SLICES), ("grid", _lib.FEM_TUNE_GRID),
+                      ("onchip_grid", _lib.FEM_TUNE_ONCHIP_GRID)):
         v = ctypes.c_int64()
         _lib.check(lib.fem_get_tuning(solver._handle, key, ctypes.byref(v)))
         out[name] = v.value
@@ -131,7 +131,10 @@ def autotune(solver, frame, restore, candidates=None, frames: int = 3, use_cache
     records = []
     for cand in candidates or DEFAULT_CANDIDATES:
         apply(solver, cand)
-        rec = {**current(solver), **measure(solver, frame, restore, frames)}
+        shape = current(solver)
+        if cand.get("onchip") == 1 and shape.get("onchip_grid") == 0:
+            continue  # it would be the streaming kernel at this candidate's shape, which is measured as such
+        rec = {**shape, **measure(solver, frame, restore, frames)}
         records.append(rec)
         if verbose:
             print(json.dumps(rec), flush=True)

@@ -62,6 +62,19 @@ def test_default_candidates_cover_every_axis():
                                            _lib.FEM_TUNE_CG_VARIANT}
 
 
+def test_the_onchip_candidate_is_measured_only_where_it_runs(monkeypatch, tmp_path):
+    cands = [dict(_cand(4, 1024), onchip=1), dict(_cand(2, 1024), onchip=0)]
+    timings = {(4, 1024, 0): 5.0, (2, 1024, 0): 9.0}
+    _patch(monkeypatch, tmp_path, timings)
+    for grid, measured in ((152, [1, 0]), (0, [0])):
+        monkeypatch.setattr(autotune, "current", lambda solver: dict(
+            solver.applied[-1], onchip_grid=grid if solver.applied[-1]["onchip"] else 0))
+        s = FakeSolver()
+        best = autotune.autotune(s, None, None, candidates=cands, use_cache=False)
+        assert [r["onchip"] for r in best["candidates"]] == measured
+        assert best["onchip"] == s.applied[-1]["onchip"] == measured[0]
+
+
 def test_operator_search_covers_batch_and_bulk_staging_and_applies_the_faster(monkeypatch):
     state = {}
 
