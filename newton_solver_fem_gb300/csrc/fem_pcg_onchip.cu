@@ -46,13 +46,9 @@ constexpr int kSmemLimit = 227 * 1024 - 1024;  // dynamic: the kernel's static v
 constexpr int kBlockBytes = 16 + 16 + 4 + 2;      // one resident block: values and local column
 constexpr int kColumnBytes = kBlockBytes * kSlice;  // one resident block column of a slice
 constexpr float kPredictFloor = 0.01f;
-// A predicted rr1 carries the sums' rounding times at most (2 / sqrt(rr1 / rr) + 1)^2: 441 at kPredictFloor, 25 at
-// kStopFloor.  So the stop is decided by the sum itself when the prediction is within kStopMargin of the
-// threshold, and the residual that a solve reports is the sum itself after a last step that cut it below
-// kStopFloor; otherwise the prediction, good to about a float unit (1.4e-7 on 5,184 Hex8 nodes at a tolerance of 0.1,
-// the sum 0.5e-7).  With a floor of 0.5 most solves paid a reduction more: 60 scenes of 125 to 729 nodes 104 us
-// against 100, 5,184 nodes 77.2 against 76.5.
-constexpr float kStopMargin = 1.01f, kStopFloor = 0.25f;
+// A predicted rr1 carries the sums' rounding times at most (2 / sqrt(rr1 / rr) + 1)^2 = 441 at that floor: within this
+// factor of the threshold it does not decide the stop, the sum itself does.
+constexpr float kStopMargin = 1.01f;
 
 // Scalars of the solve, formed by one thread from float totals (float32, like the reference's dot
 // products; FP64 is far slower here and sits on every iteration's critical path: a quotient of two
@@ -592,6 +588,7 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
         const float scale = st.scale;
         if (scale == 0.0f) {
             set_x(zero);
+            r = zero;
         } else if (scale != 1.0f) {  // a tiny right-hand side: the sums again on the normalised system
             set_x(get_x() * scale);
             r = r * scale;
@@ -674,10 +671,8 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
                 st.rr = rr1;
                 st.rz = rz;
                 st.iters += 1;
-                const bool below = rr1 <= kStopMargin * st.floor_rr;
                 st.again = rz1 < kPredictFloor * rz || rr1 < kPredictFloor * rr ||
-                           ((below || st.iters >= a.maxiter) && rr1 < kStopFloor * rr) ||
-                           (below && kStopMargin * rr1 > st.floor_rr);
+                           (rr1 <= kStopMargin * st.floor_rr && kStopMargin * rr1 > st.floor_rr);
                 st.active = (rr1 > st.floor_rr) && (st.iters < a.maxiter);
                 if (!isfinite(rr1)) {
                     st.active = 0;
@@ -686,7 +681,7 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
                 }
             });
         }
-        if (ok && st.again) {  // the predictions cancelled too far for what they decide: the sums themselves
+        if (ok && st.again) {  // the predictions cancelled, or are too close to the threshold: the sums themselves
             const float a1 = st.alpha;
             const float3 r1 = f3(fmaf(-a1, s.x, r.x), fmaf(-a1, s.y, r.y), fmaf(-a1, s.z, r.z));
             float v[8] = {dot3(r1, precondition(r1)), dot3(r1, r1), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -699,6 +694,35 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
                     atomicOr(a.status, kStatusNonFinite);
                 }
             });
+        }
+    }
+
+    // ---- the residual that is reported: the sum over the final r, not its prediction.  Nobody waits for it: a CTA
+    // leaves its part with its exit ticket, and the last one to take a ticket adds them, in a fixed order.  Both are
+    // under way while the epilogue stores (after it, behind a fence for its stores, they took 3.5 us; as one more
+    // reduction 1.7 in a cluster and 3.6 in a grid).
+    const bool several = kMeet != kAlone && team.y > 1;
+    float* const parts = a.part + ((size_t)(epoch & 1u) * gridDim.x + team.x) * 8;  // as a next reduction's
+    unsigned* const words = a.barrier + team.z * kTeamWords;
+    float rr_end = st.rr;
+    unsigned left = 0;  // the CTAs that left before this one
+    if (several) {
+        if (warp < ns) {
+            const float al = st.alpha;
+            const float3 r1 = f3(fmaf(-al, s.x, r.x), fmaf(-al, s.y, r.y), fmaf(-al, s.z, r.z));
+            const float rr = warp_sum(dot3(r1, r1));
+            if (lane == 0) red[warp] = rr;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const float rr = warp_sum(lane < ns ? red[lane] : 0.0f);
+            if (lane == 0) {
+                parts[(blockIdx.x - team.x) * 8] = rr;
+                asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
+                             : "=r"(left)
+                             : "l"(words + kTeamTicket)
+                             : "memory");
+            }
         }
     }
 
@@ -720,29 +744,30 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
             store3(a.v_out, row, v);
         }
     }
-    if (threadIdx.x == 0) {
-        if (ok && blockIdx.x == (unsigned)team.x) {
-            SceneStats o;
-            o.iterations = st.iters;
-            o.rr = st.rr;
-            o.bb = st.bb;
-            o.converged = st.rr <= st.floor_rr;
-            a.scene_stats[team.z] = o;
-            a.cum_iters[team.z] += st.iters;
-            // running max of the relative residual (non-negative floats order like their bit patterns)
-            // (a prediction may round below zero; a NaN stays one)
-            float rel = st.bb > 0.0f ? (float)sqrt((st.rr < 0.0f ? 0.0 : (double)st.rr) / (double)st.bb) : 0.0f;
-            if (!isfinite(rel)) rel = 1.0e30f;
-            atomicMax(reinterpret_cast<int*>(a.resid_max + (step_mode ? 0 : 1)), __float_as_int(rel));
-        }
-        // the team's last CTA to leave clears its barrier for the next launch: no memset per solve
-        if (kMeet == kGrid || (kMeet == kTeams && team.y > 1)) {
-            if (!ok) __threadfence();
-            unsigned* words = a.barrier + team.z * kTeamWords;
-            if (atomicAdd(words + kTeamTicket, 1u) == (unsigned)team.y - 1) {
+    if (warp == 0) {
+        const bool last = !several || __shfl_sync(0xffffffffu, left, 0) == (unsigned)team.y - 1;
+        if (several && last) {
+            __syncwarp();  // the parts that lane 0 has acquired, for every lane
+            rr_end = 0.0f;
+            for (int g = lane; g < team.y; g += 32) rr_end += __ldcg(parts + 8 * g);
+            rr_end = warp_sum(rr_end);
+            if (lane == 0) {  // and clears the team's barrier for the next launch: no memset per solve
                 words[0] = 0u;
                 words[kTeamTicket] = 0u;
             }
+        }
+        if (ok && last && lane == 0) {
+            SceneStats o;
+            o.iterations = st.iters;
+            o.rr = rr_end;
+            o.bb = st.bb;
+            o.converged = rr_end <= st.floor_rr;
+            a.scene_stats[team.z] = o;
+            a.cum_iters[team.z] += st.iters;
+            // running max of the relative residual (non-negative floats order like their bit patterns)
+            float rel = st.bb > 0.0f ? (float)sqrt((double)rr_end / (double)st.bb) : 0.0f;
+            if (!isfinite(rel)) rel = 1.0e30f;
+            atomicMax(reinterpret_cast<int*>(a.resid_max + (step_mode ? 0 : 1)), __float_as_int(rel));
         }
     }
 }
