@@ -427,6 +427,7 @@ __device__ bool reduce_across_grid(const PcgArgs& a, const Smem& sm, float* buf,
         // every partial before it is read
         if (lane == 0 && gridDim.x > 1) ok = arrive_and_wait(a.barrier, gridDim.x, epoch, a.status, a.limit_ns);
         ok = __shfl_sync(0xffffffffu, ok, 0);
+        __syncwarp();  // orders what lane 0 has acquired before the other lanes' loads (a shuffle does not)
         if (ok && S <= kWarpReducedScenes) {
             for (int sc = 0; sc < S; ++sc) {
                 const int lo = sm.sseg[sc], hi = sm.sseg[sc + 1];

@@ -297,6 +297,7 @@ __device__ __forceinline__ bool reduce8(const OcArgs& a, int4 team, float (&v)[8
             if (lane == 0) ok = arrive_and_wait(a.barrier + team.z * kTeamWords, G, epoch, a.status, a.limit_ns);
             ok = __shfl_sync(0xffffffffu, ok, 0);
             epoch = __shfl_sync(0xffffffffu, epoch, 0);
+            __syncwarp();  // orders what lane 0 has acquired before the other lanes' loads (a shuffle does not)
             if (ok) {  // lane: half (lane & 1) of the records of CTAs (lane >> 1), (lane >> 1) + 16, ...
                 const float4* b4 = reinterpret_cast<const float4*>(buf);
                 float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
