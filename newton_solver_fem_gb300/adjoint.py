@@ -10,13 +10,16 @@ converged linear solve, not of truncated CG.  One substep is
     dv  = (PAP + I - P)^-1 P rhs,   v' = v + dv,   q' = q + h v'
 
 with fixed nodes restored before the forces and after integration.  Its VJP
-(``_Substep.backward``) runs, all on the GPU through the C ABI:
+(``_Substep.backward``) is one call of the C ABI (``fem_adjoint_segment`` with one substep):
 
     vt = v'_bar + h q'_bar                    (outputs at fixed nodes carry no gradient)
-    rhs_bar = (PAP + I - P)^-1 P vt           (fem_solve: A is symmetric)
-    v_bar = vt + predictor VJP(rhs_bar)       (fem_predictor_vjp)
-    (q_bar, v_bar, a_bar, s_bar) += force VJP(h rhs_bar)   (fem_force_vjp)
+    rhs_bar = (PAP + I - P)^-1 P vt           (A is symmetric)
+    v_bar = vt + predictor VJP(rhs_bar)
+    (q_bar, v_bar, a_bar, s_bar) += force VJP(h rhs_bar)
     ext_bar = h rhs_bar
+
+The parts are also calls of their own (``fem_solve``, ``fem_predictor_vjp``, ``fem_force_vjp``;
+``DifferentiableSolver.solve`` is the first of them for a caller's own right-hand side).
 
 Beyond the reference: fixed nodes are allowed (projected solve), and a
 per-element shear scale ``s`` (``mu_scale``) is a differentiable control next
@@ -219,7 +222,12 @@ class DeviceRollout:
     segment i-1 on that handle, on its own stream, while segment i's reverse
     pass runs on the first (two state buffers alternate).  A small mesh leaves
     most SMs idle, so the recomputation comes almost for free; the two
-    cooperative PCG grids together must fit on the device, which is checked.
+    cooperative PCG grids together must fit on the device, which is checked:
+    where they do not, the recomputation is in line (``overlap`` is then None).
+    On-chip solves of more than about 77 slices (2,500 nodes) take more than
+    half the SMs; in line they are still the faster way: a 40-substep gradient of
+    2,744 Hex8 nodes takes 7.2 ms, and 13.6 with two overlapped streaming grids
+    (17,576 nodes 9.1 and 14.8).
     """
 
     def __init__(self, diff: DifferentiableSolver, steps: int, every: int, *, refresh: bool = False,

@@ -702,17 +702,16 @@ cudaError_t launch_force_vjp(Handle& h, const float* activations, const float* g
                              float* hex_mat_bar, float* ext_bar, bool accumulate, bool zero_fixed, cudaStream_t s) {
     const int acc = accumulate ? 1 : 0;
     if (h.T > 0)
-        launch_small_chained(fem::tet_force_vjp_kernel, (h.T + 127) / 128, 128, s,
-            h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.mu_scale, h.q4, h.v4, h.enable_act ? activations : nullptr, g,
-            gs, h.min_stretch, h.max_stretch, h.elem_grad, act_bar, scale_bar, tet_mat_bar, acc);
+        launch_small_chained(fem::tet_force_vjp_kernel, (h.T + 127) / 128, 128, s, h.T, h.tet_idx, h.tet_pose,
+                             h.tet_mat, h.mu_scale, h.q4, h.v4, h.enable_act ? activations : nullptr, g, gs,
+                             h.min_stretch, h.max_stretch, h.elem_grad, act_bar, scale_bar, tet_mat_bar, acc);
     if (h.H > 0)
-        launch_small_chained(fem::hex_force_vjp_kernel, (int)((8 * (int64_t)h.H + 255) / 256), 256, s,
-            h.H, h.hex_idx, h.hex_invJ, h.hex_detw, h.hex_mat, h.q4, h.v4, g, gs, h.min_stretch, h.max_stretch,
-            h.elem_grad + 2 * 4 * (size_t)h.T, hex_mat_bar, acc);
+        launch_small_chained(fem::hex_force_vjp_kernel, (int)((8 * (int64_t)h.H + 255) / 256), 256, s, h.H, h.hex_idx,
+                             h.hex_invJ, h.hex_detw, h.hex_mat, h.q4, h.v4, g, gs, h.min_stretch, h.max_stretch,
+                             h.elem_grad + 2 * 4 * (size_t)h.T, hex_mat_bar, acc);
     if (h.Tri > 0)
-        launch_small_chained(fem::tri_force_vjp_kernel, (h.Tri + 127) / 128, 128, s,
-            h.Tri, h.tri_idx, h.tri_pose, h.tri_mat, h.q4, h.v4, g, gs,
-            h.elem_grad + 2 * (4 * (size_t)h.T + 8 * (size_t)h.H));
+        launch_small_chained(fem::tri_force_vjp_kernel, (h.Tri + 127) / 128, 128, s, h.Tri, h.tri_idx, h.tri_pose,
+                             h.tri_mat, h.q4, h.v4, g, gs, h.elem_grad + 2 * (4 * (size_t)h.T + 8 * (size_t)h.H));
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     fem::NodeVjpArgs a;
@@ -750,18 +749,16 @@ cudaError_t launch_force_vjp(Handle& h, const float* activations, const float* g
     a.ext_bar = ext_bar;
     a.q_bar = q_bar;
     a.v_bar = v_bar;
-    launch_small_chained(fem::node_vjp_kernel, (h.P + 127) / 128, 128, s,
-            a);
+    launch_small_chained(fem::node_vjp_kernel, (h.P + 127) / 128, 128, s, a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_predictor_vjp(Handle& h, const float* rhs_bar, float dt, float* v_bar, cudaStream_t s) {
     const int threads = 256;
     const int blocks = (h.nslices * 32 + threads - 1) / threads;
-    launch_small_chained(fem::predictor_vjp_kernel, blocks, threads, s,
-            h.nslices, h.slice_ptr, h.slice_meta, h.row_info, h.valA,
-                                                          h.valB, h.valC, h.scol, rhs_bar, h.node_spring_ptr,
-                                                          h.node_spring_ent, h.spring_idx, h.spring_kd, dt, v_bar);
+    launch_small_chained(fem::predictor_vjp_kernel, blocks, threads, s, h.nslices, h.slice_ptr, h.slice_meta,
+                         h.row_info, h.valA, h.valB, h.valC, h.scol, rhs_bar, h.node_spring_ptr, h.node_spring_ent,
+                         h.spring_idx, h.spring_kd, dt, v_bar);
     return cudaGetLastError();
 }
 
@@ -909,12 +906,11 @@ int fem_adjoint_segment(FemHandle* H, float* q_states, float* v_states, int32_t 
     cudaError_t err = refresh ? refresh_at(h, q_states, s) : cudaSuccess;
     float* rb = adjoint_start != nullptr ? adjoint_start : h.adj_x;  // the adjoint solution (and warm start)
     for (int k = substeps - 1; k >= 0 && err == cudaSuccess; --k) {
-        launch_small_chained(fem::adjoint_seed_kernel, blocks, threads, s,
-            h.P, dt, h.fixed_mask, q_bar, v_bar, h.adj_vt);
+        launch_small_chained(fem::adjoint_seed_kernel, blocks, threads, s, h.P, dt, h.fixed_mask, q_bar, v_bar,
+                             h.adj_vt);
         err = cudaGetLastError();
         if (err == cudaSuccess && adjoint_start != nullptr) {
-            launch_small_chained(fem::pack_adjoint_start_kernel, blocks, threads, s,
-            h.P, rb, h.fixed_mask, h.x);
+            launch_small_chained(fem::pack_adjoint_start_kernel, blocks, threads, s, h.P, rb, h.fixed_mask, h.x);
             err = cudaGetLastError();
         }
         if (err == cudaSuccess)

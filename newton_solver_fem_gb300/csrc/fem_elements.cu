@@ -585,14 +585,14 @@ __global__ void __launch_bounds__(kTetTangentThreads) tet_tangent_kernel(
 //            records r of its point (no work repeated across lanes);
 //   phase 2  one thread per 2x2 tile of blocks on or above the block diagonal (10 tiles per
 //            hex) sums its four blocks over the 8 points (K_ba = K_ab^T term by term, so the
-//            blocks below the diagonal are not formed and A is exactly symmetric).  Threads are tile-major (16 hexes per tile), so a quarter
-//            warp reads 8 hexes' records in 8 distinct bank groups and a diagonal tile's half
-//            warp skips its column-side loads;
+//            blocks below the diagonal are not formed and A is exactly symmetric).  Threads are
+//            tile-major (16 hexes per tile), so a quarter warp reads 8 hexes' records in 8 distinct
+//            bank groups and a diagonal tile's half warp skips its column-side loads;
 //   phase 3  the 36 blocks per hex are staged in shared memory in the triplet planes' layout (block by
 //            block over the group's 16 hexes, so a half warp stores one run) and written out by one
 //            bulk asynchronous copy (cp.async.bulk) per plane.
 // 48^3 hexes: 105 us writing all 64 blocks a hex, 80 writing 36 (143 MB); what bounds it is shared
-// memory (about 2,000 wavefronts a CTA, 47 us) and issue (about 7,500 instructions, 44 us) together.
+// memory (2,375 wavefronts a CTA, 52 us) and issue (7,530 warp instructions, 41 us) together.
 constexpr int kTanHex = kHexGroup;
 constexpr int kTanTiles = 10;
 constexpr int kTanThreads = kTanHex * kTanTiles;
@@ -970,17 +970,17 @@ cudaError_t launch_constant_blocks(Handle& h, float dt, cudaStream_t s) {
 
 cudaError_t launch_element_tangent(Handle& h, float dt, cudaStream_t s) {
     if (h.T > 0)
-        launch_maybe_chained(
-            blocks_for(h.T, kTetTangentThreads) <= (int)kChainedBlocks, tet_tangent_kernel,
-            blocks_for(h.T, kTetTangentThreads), kTetTangentThreads, 0, s, h.T, h.tet_idx, h.tet_pose, h.tet_mat, h.mu_scale, h.q4, h.min_stretch, h.max_stretch, dt,
-            h.trip_map.tet_start(), h.trip);
+        launch_maybe_chained(blocks_for(h.T, kTetTangentThreads) <= (int)kChainedBlocks, tet_tangent_kernel,
+                             blocks_for(h.T, kTetTangentThreads), kTetTangentThreads, 0, s, h.T, h.tet_idx, h.tet_pose,
+                             h.tet_mat, h.mu_scale, h.q4, h.min_stretch, h.max_stretch, dt, h.trip_map.tet_start(),
+                             h.trip);
     if (h.H > 0) {
         cudaError_t err = allow_dynamic_smem((const void*)hex_tangent_kernel, kTanSmemBytes);
         if (err != cudaSuccess) return err;
-        launch_maybe_chained(
-            blocks_for(h.H, kTanHex) <= (int)kChainedBlocks, hex_tangent_kernel, blocks_for(h.H, kTanHex), kTanThreads,
-            kTanSmemBytes, s, h.H, h.hex_idx, h.hex_invJ, h.hex_detw, h.hex_mat, h.q4, h.min_stretch, h.max_stretch, dt,
-            h.trip_map.hex_start(), h.trip);
+        launch_maybe_chained(blocks_for(h.H, kTanHex) <= (int)kChainedBlocks, hex_tangent_kernel,
+                             blocks_for(h.H, kTanHex), kTanThreads, kTanSmemBytes, s, h.H, h.hex_idx, h.hex_invJ,
+                             h.hex_detw, h.hex_mat, h.q4, h.min_stretch, h.max_stretch, dt, h.trip_map.hex_start(),
+                             h.trip);
     }
     return cudaGetLastError();
 }

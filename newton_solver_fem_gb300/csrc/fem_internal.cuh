@@ -81,8 +81,10 @@ __device__ __forceinline__ void store_block(const TripletPlanes& t, int64_t i, c
 // the stream's, as before; what goes is the launch latency between two short kernels (eagerly and in
 // captured graphs): a substep's five launches take 10 us less.  A kernel launched this way begins with
 // chained_start().  The tangent and the assembly are chained only while their grid is at most
-// kChainedBlocks: a 1,500-CTA assembly behind an early start, with device copies after it, made the
-// refresh and export of 26,220 Tet4 nodes 125 us instead of 84 (and 48^3 Hex8 251 instead of 230).
+// kChainedBlocks, twice the SM count: a 1,500-CTA assembly behind an early start, with device copies after
+// it, made the refresh and export of 26,220 Tet4 nodes 125 us instead of 84 (and 48^3 Hex8 251 instead of
+// 230).  That is the line for a refresh that copies follow.  The export has no copies of its own any more; right
+// before it, chaining at every size measures 41 instead of 44 us there (15,625 Hex8 nodes 34 and 37, 32^3 74 and 75).
 #ifdef __CUDACC__
 __device__ __forceinline__ void chained_start() {
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");

@@ -30,10 +30,12 @@
 // Every sum has a fixed order and every CTA forms bit-identical totals.
 //
 // Measured, us per iteration (50-iteration solves, launch included), streaming kernel -> this one:
-//   Tet4 425 nodes 8.3 -> 2.1, 1,000 12.5 -> 2.3, 4,913 10.1 -> 3.6, 15,625 10.6 -> 3.8, 50,653
-//   11.5 -> 5.5, 117,649 14.8 -> 10.2; Hex8 1,000 16.6 -> 2.4, 5,184 13.1 -> 3.8, 35,937 13.4 -> 5.7,
-//   68,921 15.5 -> 9.0, 117,649 30.7 -> 21.8.  What remains is the barrier (2.4 us of a grid, 1.0 of a
-//   cluster) and, from 30,000 nodes, the wavefronts of the product and the columns read from L2.
+//   Tet4 8 nodes 4.2 -> 0.85, 81 6.9 -> 1.2, 425 8.4 -> 2.4, 1,000 11.4 -> 2.4, 4,913 10.3 -> 3.7, 15,625 10.5 -> 4.1,
+//   50,653 11.2 -> 5.7, 117,649 13.5 -> 10.1, 151,686 19.8 -> 13.2; Hex8 27 nodes 9.4 -> 1.2, 1,000 14.5 -> 2.6, 5,184
+//   13.4 -> 3.9, 24,389 13.2 -> 4.8, 35,937 13.2 -> 5.8, 51,578 14.0 -> 7.4, 68,921 14.4 -> 8.8, 117,649 25.5..27.5 -> 21.6.
+// What remains is the meeting (2.4 us of a grid, 1.0 of a cluster): at 5,184 Hex8 nodes most warps wait at the CTA
+// barrier that follows it, 11% of the issue slots and 10% of the shared-memory pipe are used.  From 30,000 nodes come
+// the columns read from L2: 44 MB an iteration at 68,921 nodes, where the product's shared wavefronts take 2 us.
 #include <algorithm>
 #include <vector>
 
@@ -764,7 +766,8 @@ __global__ void __launch_bounds__(kThreads, 1) onchip_pcg_kernel(OcArgs a) {
             o.bb = st.bb;
             o.converged = rr_end <= st.floor_rr;
             a.scene_stats[team.z] = o;
-            a.cum_iters[team.z] += st.iters;
+            // an atomic has no load to wait for at the kernel's end (0.3 us)
+            atomicAdd(reinterpret_cast<unsigned long long*>(a.cum_iters + team.z), (unsigned long long)st.iters);
             // running max of the relative residual (non-negative floats order like their bit patterns)
             float rel = st.bb > 0.0f ? (float)sqrt((double)rr_end / (double)st.bb) : 0.0f;
             if (!isfinite(rel)) rel = 1.0e30f;
@@ -779,9 +782,10 @@ using OcKernel = void (*)(OcArgs);
 // gather, a shared one fourteen; 5, 6 and 7 blocks spill: 3.9, 4.3 and 4.7 us per iteration against 3.8
 // on 5,184 nodes); more slices (one owner thread per row) in 1024 threads of 64.
 constexpr int kOcRegs = 4, kOcWideWarps = 16;
-// Where the launches cross, in stored block columns of all slices (us per iteration on GB300):
-//   alone 1.1 (27 nodes) to 2.0 at 128 columns, a cluster 2.0 from there (Tet4 8 slices, 120 columns:
-//   1.81 alone, 1.97 in 8 CTAs; Hex8 6 slices, 162 columns: 2.14 and 2.01);
+// Where the launches cross, in stored block columns of all slices (us per iteration on GB300, one CTA and a cluster):
+//   Hex8 27 nodes (27 columns) 1.2 and 1.9, Tet4 180 (90) 1.7 and 2.1, Hex8 125 (108) 1.7 and 2.3, Tet4 252 (120) 1.8
+//   and 2.1, Hex8 150 (135) 1.8 and 2.3, Hex8 180 (162) 2.1 and 2.2, Tet4 448 (210) 2.3 and 2.4, Hex8 245 (216) 2.45
+//   and 2.3: the crossing is near 200, and the line, at 128, is where every body measured is faster alone;
 //   a cluster of 16 reaches a grid's 3.4 near 2,000 columns (Hex8 74 slices, 1,998 columns: 3.22 and
 //   3.39; Tet4 106 slices, 1,590: 3.16 and 3.34; Hex8 106 slices, 2,862: 3.85 and 3.47).
 constexpr int64_t kAloneColumns = 128, kClusterColumns = 2000;

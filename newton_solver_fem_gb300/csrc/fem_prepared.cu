@@ -497,7 +497,8 @@ int fem_prepared_solve(FemHandle* H, const FemPreparedWs* w, const float* rhs, f
     if (h.P == 0) return FEM_OK;
     fem::Guard g(H->device);
     cudaStream_t s = (cudaStream_t)stream;
-    fem::launch_chained(fem::pack_warm_start_kernel, fem::blocks(h.P, 256), 256, 0, s, h.P, w->increment, h.fixed_mask, h.x);
+    fem::launch_chained(fem::pack_warm_start_kernel, fem::blocks(h.P, 256), 256, 0, s, h.P, w->increment, h.fixed_mask,
+                        h.x);
     cudaError_t err = cudaGetLastError();
     if (err == cudaSuccess)
         err = fem::launch_pcg(h, dt, 0, nullptr, nullptr, nullptr, s, rhs, w->increment, tolerance, maxiter,
@@ -514,7 +515,8 @@ int fem_prepared_reconstruct(FemHandle* H, const FemPreparedWs* w, const float* 
     Handle& h = H->h;
     if (h.P == 0) return FEM_OK;
     fem::Guard g(H->device);
-    fem::launch_chained(fem::reconstruct_kernel, fem::blocks(h.P, 256), 256, 0, (cudaStream_t)stream, h.P, dv, w->q, w->v, h.fixed_mask, h.rest, dt, q_out, v_out);
+    fem::launch_chained(fem::reconstruct_kernel, fem::blocks(h.P, 256), 256, 0, (cudaStream_t)stream, h.P, dv, w->q,
+                        w->v, h.fixed_mask, h.rest, dt, q_out, v_out);
     return fem::report_cuda(cudaGetLastError());
 }
 
